@@ -192,9 +192,8 @@ zsmpm_status allocate_particles(zsmpm_scene *s, int64_t cap) {
   for (int k = 0; k < 2; ++k) {
     particle_buffers &b = s->bufs[k];
     ZS_ALLOC(b.xm, cap, "alloc xm");
-    ZS_ALLOC(b.v, cap, "alloc v");
+    ZS_ALLOC(b.row, 3 * mat_capacity(cap), "alloc rows");
     ZS_ALLOC(b.C, 9 * mat_capacity(cap), "alloc C");
-    ZS_ALLOC(b.A, 9 * mat_capacity(cap), "alloc A");
     ZS_ALLOC(b.F, 9 * mat_capacity(cap), "alloc F");
     if (plastic) ZS_ALLOC(b.plastic, cap, "alloc plastic");
     ZS_ALLOC(b.id, cap, "alloc id");
@@ -312,12 +311,15 @@ constexpr int kGraphSubsteps = 4;
 // defer_closure: with a learned closure attached, leave the closure pass (network and finish)
 // to the side stream and have the next substep_enqueue join it before its P2G (zsmpm_run's
 // graphs only; the side stream and its events must exist)
-zsmpm_status substep_enqueue(zsmpm_scene *s, cudaStream_t st, bool defer_closure = false) {
+// store_c: whether G2P stores C.  P2G takes the affine momentum and the next G2P overwrites C, so of
+// the substeps of one call only the last one's C can be read (G2P's stores 149 -> 113 bytes a
+// particle in the others).
+zsmpm_status substep_enqueue(zsmpm_scene *s, cudaStream_t st, bool defer_closure = false, bool store_c = true) {
   bind_buffers(s);
   if (s->timing) cudaEventRecord(s->ev[0], st);
+  s->dev.prm.bin_full = 0;
   ZS_TRY(launch_activate(s->dev, st), "activate");
   if (s->timing) cudaEventRecord(s->ev[1], st);
-  s->dev.prm.bin_full = 0;
   ZS_TRY(launch_bin(s->dev, st), "bin");
   if (s->timing) cudaEventRecord(s->ev[2], st);
   if (s->join_pending) {
@@ -331,7 +333,10 @@ zsmpm_status substep_enqueue(zsmpm_scene *s, cudaStream_t st, bool defer_closure
   ZS_TRY(launch_grid_update(s->dev, st), "grid update");
   if (s->timing) cudaEventRecord(s->ev[4], st);
   const bool deferred = defer_closure && s->dev.aux.learned && s->side_stream;
-  ZS_TRY(launch_g2p(s->dev, st, !deferred), "g2p");
+  s->dev.prm.store_c = store_c ? 1 : 0;
+  const cudaError_t g2p = launch_g2p(s->dev, st, !deferred);
+  s->dev.prm.store_c = 1;
+  ZS_TRY(g2p, "g2p");
   if (deferred) {
     ZS_TRY(cudaEventRecord(s->fork_ev, st), "fork the closure pass");
     ZS_TRY(cudaStreamWaitEvent(s->side_stream, s->fork_ev, 0), "fork the closure pass");
@@ -402,6 +407,7 @@ ZSMPM_API zsmpm_status zsmpm_scene_create(const zsmpm_scene_desc *desc, zsmpm_sc
   p.wall_cells = desc->wall_cells;
   p.mat = make_material(desc->material);
   p.g2p_threads = desc->threads_per_cta;
+  p.store_c = 1;
   for (auto &ev : s->ev) cudaEventCreate(&ev);
   e = prepare_kernels();
   if (e != cudaSuccess) {
@@ -852,7 +858,7 @@ ZSMPM_API zsmpm_status zsmpm_run(zsmpm_scene *s, int32_t nsteps, void *stream) {
     ZS_TRY(cudaStreamBeginCapture(s->graph_stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     zsmpm_status a = ZSMPM_OK;
     for (int k = 0; k < kGraphSubsteps && a == ZSMPM_OK; ++k)
-      a = substep_enqueue(s, s->graph_stream, k + 1 < kGraphSubsteps);
+      a = substep_enqueue(s, s->graph_stream, k + 1 < kGraphSubsteps, k + 1 == kGraphSubsteps);
     s->join_pending = false;  // the last substep joined the pass before it (or capture failed)
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s->graph_stream, &g);
@@ -884,7 +890,7 @@ ZSMPM_API zsmpm_status zsmpm_run(zsmpm_scene *s, int32_t nsteps, void *stream) {
   }
   // an even number of substeps leaves the parity unchanged
   for (; done < nsteps; ++done) {
-    st = substep_enqueue(s, cs);
+    st = substep_enqueue(s, cs, false, done + 1 == nsteps);
     if (st != ZSMPM_OK) {
       s->timing = timing;
       return st;
@@ -1024,7 +1030,9 @@ ZSMPM_API zsmpm_status zsmpm_stage_times(zsmpm_scene *s, float *ms, int32_t coun
   return ZSMPM_OK;
 }
 
-ZSMPM_API int32_t zsmpm_kernels_per_substep(const zsmpm_scene *) { return kernels_per_substep(); }
+ZSMPM_API int32_t zsmpm_kernels_per_substep(const zsmpm_scene *s) {
+  return kernels_per_substep(s ? s->dev : scene_device{});
+}
 
 ZSMPM_API zsmpm_status zsmpm_scene_set_closure(zsmpm_scene *s, zsmpm_closure *c, int32_t audit_period) {
   zsmpm_status st = check_scene(s, false);

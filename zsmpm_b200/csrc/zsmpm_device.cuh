@@ -72,6 +72,14 @@ constexpr float kFourGammaSq = 5.8284273147583007813f;
 __device__ __forceinline__ float sin_pi8() { return __int_as_float(1053028117); }
 __device__ __forceinline__ float cos_pi8() { return __int_as_float(1064076127); }
 
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// kScale: the reference's rescaling of the matrix by the rotation's rounded norm
+template <bool kScale = true>
 __device__ __forceinline__ void conjugate(float &pp, float &qq, float &rr, float &pq, float &rp,
                                           float &rq, float &qs, float &qk, float &qi,
                                           float &qj) {
@@ -81,7 +89,8 @@ __device__ __forceinline__ void conjugate(float &pp, float &qq, float &rr, float
   sh = big ? sh : 0.f;
   float ch = big ? t5 : 1.f;
   float sh2 = sh * sh, ch2 = ch * ch;
-  const float r = rsqrtf(sh2 + ch2);
+  // (sh2 + ch2 is 1e-20 or more, so no subnormals)
+  const float r = kScale ? rsqrtf(sh2 + ch2) : rsqrt_ftz(sh2 + ch2);
   sh *= r;
   ch *= r;
   if (ch2 <= kFourGammaSq * sh2) {
@@ -92,10 +101,12 @@ __device__ __forceinline__ void conjugate(float &pp, float &qq, float &rr, float
   ch2 = ch * ch;
   const float c = ch2 - sh2;
   const float s = 2.f * ch * sh;
-  const float scale = sh2 + ch2;
-  rr = rr * scale * scale;
-  rp *= scale;
-  rq *= scale;
+  if (kScale) {
+    const float scale = sh2 + ch2;
+    rr = rr * scale * scale;
+    rp *= scale;
+    rq *= scale;
+  }
   const float rp0 = rp, rq0 = rq;
   rp = c * rp0 + s * rq0;
   rq = c * rq0 - s * rp0;
@@ -179,11 +190,11 @@ __device__ __forceinline__ void swap_cols(float a[3][3], float v[3][3], float rh
 
 // A (column-major) = U diag(S) V^T; U, V rotations; S sorted by magnitude, S[2] may be < 0.
 // kWarpEarlyExit: stop the Jacobi sweeps after the second or third once, for every lane of the
-// warp, the off-diagonal of A^T A is below 1e-7 of its diagonal (squared: 1e-14), where the
-// remaining sweeps only move the result by rounding.  Every lane of the warp must call it then.
-// The default runs the reference's four sweeps.
+// call, the off-diagonal of A^T A is below 1e-7 of its diagonal (squared: 1e-14), where the
+// remaining sweeps only move the result by rounding.  `lanes` are then the lanes of the warp that
+// call it together.  The default runs the reference's four sweeps.
 template <bool kWarpEarlyExit = false>
-__device__ __forceinline__ void svd3(const float *A, float *U, float *S, float *V) {
+__device__ __forceinline__ void svd3(const float *A, float *U, float *S, float *V, unsigned lanes = 0xffffffffu) {
   using namespace svd_detail;
   float a[3][3];
 #pragma unroll
@@ -202,7 +213,7 @@ __device__ __forceinline__ void svd3(const float *A, float *U, float *S, float *
     if (kWarpEarlyExit && sweep >= 2) {
       const float off = s21 * s21 + s31 * s31 + s32 * s32;
       const float diag = s11 * s11 + s22 * s22 + s33 * s33;
-      if (__all_sync(0xffffffffu, off <= 1e-14f * diag)) break;
+      if (__all_sync(lanes, off <= 1e-14f * diag)) break;
     }
     conjugate(s11, s22, s33, s21, s31, s32, qs, qz, qx, qy);
     conjugate(s22, s33, s11, s32, s21, s31, qs, qx, qy, qz);
@@ -258,6 +269,79 @@ __device__ __forceinline__ void svd3(const float *A, float *U, float *S, float *
   S[0] = a[0][0];
   S[1] = a[1][1];
   S[2] = a[2][2];
+}
+
+// A = U diag(S) V^T for an A whose singular values are of similar size (det A > 0 and none below a
+// tenth of the largest, else false): the Jacobi sweeps above for V, then the columns of A V
+// normalised in place of the sort and the Givens QR, which an isotropic model has no use for (it
+// takes the singular values in any order).  About 480 instructions against about 700, and U is
+// orthonormal to half the QR's error (which drops elements below 1e-6).  The Jacobi matrix is
+// not rescaled after each rotation: that only matters to V's scale through rounding.
+// kWarpEarlyExit as in svd3.
+template <bool kWarpEarlyExit = false>
+__device__ __forceinline__ bool svd3_columns(const float *A, float *U, float *S, float *V, unsigned lanes = 0xffffffffu) {
+  using namespace svd_detail;
+  float s11 = A[0] * A[0] + A[1] * A[1] + A[2] * A[2];
+  float s21 = A[3] * A[0] + A[4] * A[1] + A[5] * A[2];
+  float s31 = A[6] * A[0] + A[7] * A[1] + A[8] * A[2];
+  float s22 = A[3] * A[3] + A[4] * A[4] + A[5] * A[5];
+  float s32 = A[6] * A[3] + A[7] * A[4] + A[8] * A[5];
+  float s33 = A[6] * A[6] + A[7] * A[7] + A[8] * A[8];
+  float qs = 1.f, qx = 0.f, qy = 0.f, qz = 0.f;
+#pragma unroll
+  for (int sweep = 0; sweep < 4; ++sweep) {
+    if (kWarpEarlyExit && sweep >= 2) {
+      const float off = s21 * s21 + s31 * s31 + s32 * s32;
+      const float diag = s11 * s11 + s22 * s22 + s33 * s33;
+      if (__all_sync(lanes, off <= 1e-14f * diag)) break;
+    }
+    conjugate<false>(s11, s22, s33, s21, s31, s32, qs, qz, qx, qy);
+    conjugate<false>(s22, s33, s11, s32, s21, s31, qs, qx, qy, qz);
+    conjugate<false>(s33, s11, s22, s31, s32, s21, qs, qy, qz, qx);
+  }
+  {
+    const float n2 = qs * qs + qx * qx + qy * qy + qz * qz;
+    const float y = __frsqrt_rn(n2);
+    const float r = fmaf(-n2, 0.5f * y * y * y, fmaf(0.5f, y, y));  // one Newton step, as refined_rsqrt
+    qs *= r;
+    qx *= r;
+    qy *= r;
+    qz *= r;
+  }
+  const float xx = qx * qx, yy = qy * qy, zz = qz * qz, ww = qs * qs;
+  const float x2 = qx + qx, y2 = qy + qy, z2 = qz + qz;
+  const float wx = qs * x2, wy = qs * y2, wz = qs * z2;
+  const float xy = qy * x2, yz = qz * y2, zx = qx * z2;
+  V[0] = ww + xx - yy - zz;
+  V[4] = ww - xx + yy - zz;
+  V[8] = ww - xx - yy + zz;
+  V[3] = xy - wz;
+  V[7] = yz - wx;
+  V[2] = zx - wy;
+  V[1] = xy + wz;
+  V[5] = yz + wx;
+  V[6] = zx + wy;
+  float lo = 3.4e38f, hi = 0.f;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float b0 = A[0] * V[3 * c] + A[3] * V[3 * c + 1] + A[6] * V[3 * c + 2];
+    const float b1 = A[1] * V[3 * c] + A[4] * V[3 * c + 1] + A[7] * V[3 * c + 2];
+    const float b2 = A[2] * V[3 * c] + A[5] * V[3 * c + 1] + A[8] * V[3 * c + 2];
+    const float rho = b0 * b0 + b1 * b1 + b2 * b2;
+    // sqrt(rho) and its reciprocal, each with one Newton step
+    const float y = rsqrtf(rho), q = rho * y;
+    const float r = fmaf(0.5f * y, fmaf(-q, y, 1.f), y);
+    lo = fminf(lo, rho);
+    hi = fmaxf(hi, rho);
+    S[c] = fmaf(0.5f * y, fmaf(-q, q, rho), q);
+    U[3 * c] = b0 * r;
+    U[3 * c + 1] = b1 * r;
+    U[3 * c + 2] = b2 * r;
+  }
+  // (a NaN fails)
+  const float det = A[0] * (A[4] * A[8] - A[7] * A[5]) + A[3] * (A[7] * A[2] - A[1] * A[8]) +
+                    A[6] * (A[1] * A[5] - A[4] * A[2]);
+  return det > 0.f && lo >= 0.01f * hi && lo > 1e-30f && hi < 1e30f;
 }
 
 // ---------------------------------------------------------------- constitutive models
@@ -505,12 +589,24 @@ __device__ __forceinline__ void mul_diag_t(float *out, const float *M, const flo
       out[3 * c + r] = M[r] * d[0] * N[c] + M[3 + r] * d[1] * N[3 + c] + M[6 + r] * d[2] * N[6 + c];
 }
 
+// U diag(d) U^T
+__device__ __forceinline__ void mul_diag_sym(float *out, const float *U, const float *d) {
+  float W[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) W[k] = U[k] * d[k / 3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int r = 0; r <= c; ++r)
+      out[3 * c + r] = out[3 * r + c] = W[r] * U[c] + W[3 + r] * U[3 + c] + W[6 + r] * U[6 + c];
+}
+
 // Kirchhoff stress tau = V0 P F^T for an isotropic model with F = U diag(S) V^T and
 // principal first Piola stress Ph: P F^T = U diag(Ph * S) U^T.
 __device__ __forceinline__ void kirchhoff(float *tau, const float *U, const float *Ph,
                                           const float *S, float volume) {
   const float d[3] = {Ph[0] * S[0] * volume, Ph[1] * S[1] * volume, Ph[2] * S[2] * volume};
-  mul_diag_t(tau, U, d, U);
+  mul_diag_sym(tau, U, d);
 }
 
 // Fixed corotated principal stress (ConstitutiveModel_Vol_dP.hpp:17-23)
@@ -522,14 +618,23 @@ __device__ __forceinline__ void fc_principal(float mu, float lambda, const float
   Ph[2] = smu * (S[2] - 1.f) + sl * (S[0] * S[1]);
 }
 
+__device__ __forceinline__ void constitutive_principal(const material_dev &mat, const float *U, const float *S,
+                                                       const float *V, float *F, float &plastic, float *tau);
+
 // Return map + stress.  F: trial deformation in, F after the model's projection out
 // (the projected F is what the reference's stress functions leave in their F argument);
 // plastic: logJp (DP) or Jp (snow); tau out.  Reference ordering keeps F unchanged.
 template <bool kWarpEarlyExit = false>
 __device__ __forceinline__ void constitutive(const material_dev &mat, float *F, float &plastic,
-                                             float *tau) {
+                                             float *tau, unsigned lanes = 0xffffffffu) {
   float U[9], S[3], V[9];
-  svd3<kWarpEarlyExit>(F, U, S, V);
+  svd3<kWarpEarlyExit>(F, U, S, V, lanes);
+  constitutive_principal(mat, U, S, V, F, plastic, tau);
+}
+
+// The update from the trial F = U diag(S) V^T
+__device__ __forceinline__ void constitutive_principal(const material_dev &mat, const float *U, const float *S,
+                                                       const float *V, float *F, float &plastic, float *tau) {
   if (mat.model == 0) {
     float Ph[3];
     fc_principal(mat.mu, mat.lambda, S, Ph);
@@ -574,7 +679,7 @@ __device__ __forceinline__ void constitutive(const material_dev &mat, float *F, 
     float PhNs[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) PhNs[i] = (smu * logNs[i] + mat.lambda * trl) * mat.volume;
-    mul_diag_t(tau, U, PhNs, U);
+    mul_diag_sym(tau, U, PhNs);
   } else {
     // snow: SnowPlasticity::do_project_sigma (SnowPlasticity.hpp:24-32) committed to F,
     // Jp accumulated, then fixed corotated with hardened Lame parameters
@@ -590,6 +695,156 @@ __device__ __forceinline__ void constitutive(const material_dev &mat, float *F, 
     kirchhoff(tau, U, Ph, Ns, mat.volume);
   }
   if (mat.mode == 0) mul_diag_t(F, U, Ns, V);
+}
+
+// ---------------------------------------------------------------- small strains without an SVD
+// Fixed corotated stress is an isotropic function of b = F F^T = I + E, so where the strain is small it
+// follows from a power series of symmetric matrices, without singular values:
+//   Z = E (2 I + E)^-1,   sqrt(b) = ((I + Z) / (I - Z))^(1/2) = (I + Z)(I + Z^2/2 + 3 Z^4/8 + ...),
+// with the powers reduced to c2 Z^2 + c1 Z + c0 I by Cayley-Hamilton (Z^3 = i1 Z^2 - i2 Z + i3),
+// three operations a power.  E carries the rounding of F F^T alone and the series is cut below
+// FP32 rounding, so the stress is closer to the exact one than that of the Jacobi SVD.  About 190
+// instructions against about 750.
+struct sym3 {
+  float xx, yy, zz, xy, xz, yz;
+};
+
+__device__ __forceinline__ float det3(const float *F) {
+  return F[0] * (F[4] * F[8] - F[7] * F[5]) + F[3] * (F[7] * F[2] - F[1] * F[8]) + F[6] * (F[1] * F[5] - F[4] * F[2]);
+}
+
+__device__ __forceinline__ sym3 sym_square(const sym3 &a) {
+  sym3 r;
+  r.xx = a.xx * a.xx + a.xy * a.xy + a.xz * a.xz;
+  r.yy = a.xy * a.xy + a.yy * a.yy + a.yz * a.yz;
+  r.zz = a.xz * a.xz + a.yz * a.yz + a.zz * a.zz;
+  r.xy = a.xx * a.xy + a.xy * a.yy + a.xz * a.yz;
+  r.xz = a.xx * a.xz + a.xy * a.yz + a.xz * a.zz;
+  r.yz = a.xy * a.xz + a.yy * a.yz + a.yz * a.zz;
+  return r;
+}
+
+__device__ __forceinline__ float sym_det(const sym3 &a) {
+  return a.xx * (a.yy * a.zz - a.yz * a.yz) + a.xy * (a.xz * a.yz - a.xy * a.zz) + a.xz * (a.xy * a.yz - a.xz * a.yy);
+}
+
+// c2 A^2 + c1 A + c0 I
+__device__ __forceinline__ sym3 sym_poly(const sym3 &a2, const sym3 &a, float c2, float c1, float c0) {
+  sym3 r;
+  r.xx = c2 * a2.xx + (c1 * a.xx + c0);
+  r.yy = c2 * a2.yy + (c1 * a.yy + c0);
+  r.zz = c2 * a2.zz + (c1 * a.zz + c0);
+  r.xy = c2 * a2.xy + c1 * a.xy;
+  r.xz = c2 * a2.xz + c1 * a.xz;
+  r.yz = c2 * a2.yz + c1 * a.yz;
+  return r;
+}
+
+// powers A^n = p.c2 A^2 + p.c1 A + p.c0 I by the invariants of A
+struct sym_power {
+  float c2, c1, c0;
+  __device__ __forceinline__ void next(float i1, float i2, float i3) {
+    const float q = c2;
+    c2 = i1 * q + c1;
+    c1 = c0 - i2 * q;
+    c0 = i3 * q;
+  }
+};
+
+// the strain measures of a trial F: E, Z, Z^2 and Z's invariants; t2 = tr Z^2
+struct small_strain {
+  sym3 E, Z, Z2;
+  float i1, i2, i3, t2;
+};
+
+__device__ __forceinline__ void strain_of(const float *F, small_strain &s) {
+  sym3 &E = s.E, &Z = s.Z;
+  E.xx = F[0] * F[0] + (F[3] * F[3] + (F[6] * F[6] - 1.f));
+  E.yy = F[1] * F[1] + (F[4] * F[4] + (F[7] * F[7] - 1.f));
+  E.zz = F[2] * F[2] + (F[5] * F[5] + (F[8] * F[8] - 1.f));
+  E.xy = F[0] * F[1] + F[3] * F[4] + F[6] * F[7];
+  E.xz = F[0] * F[2] + F[3] * F[5] + F[6] * F[8];
+  E.yz = F[1] * F[2] + F[4] * F[5] + F[7] * F[8];
+  const float mx = 2.f + E.xx, my = 2.f + E.yy, mz = 2.f + E.zz;
+  sym3 c;  // cofactors of 2 I + E
+  c.xx = my * mz - E.yz * E.yz;
+  c.yy = mx * mz - E.xz * E.xz;
+  c.zz = mx * my - E.xy * E.xy;
+  c.xy = E.xz * E.yz - E.xy * mz;
+  c.xz = E.xy * E.yz - E.xz * my;
+  c.yz = E.xy * E.xz - E.yz * mx;
+  const float inv = __fdividef(1.f, mx * c.xx + E.xy * c.xy + E.xz * c.xz);
+  Z.xx = (E.xx * c.xx + E.xy * c.xy + E.xz * c.xz) * inv;
+  Z.yy = (E.xy * c.xy + E.yy * c.yy + E.yz * c.yz) * inv;
+  Z.zz = (E.xz * c.xz + E.yz * c.yz + E.zz * c.zz) * inv;
+  Z.xy = (E.xx * c.xy + E.xy * c.yy + E.xz * c.yz) * inv;
+  Z.xz = (E.xx * c.xz + E.xy * c.yz + E.xz * c.zz) * inv;
+  Z.yz = (E.xy * c.xz + E.yy * c.yz + E.yz * c.zz) * inv;
+  s.Z2 = sym_square(Z);
+  s.i1 = Z.xx + Z.yy + Z.zz;
+  s.t2 = s.Z2.xx + s.Z2.yy + s.Z2.zz;
+  s.i2 = 0.5f * (s.i1 * s.i1 - s.t2);
+  s.i3 = sym_det(Z);
+}
+
+// sqrt(b) - I, for |Z|_F <= 0.2 (the next term, 0.25 Z^10, is below 2.5e-8)
+constexpr float kSmallRoot2 = 0.04f;
+__device__ __forceinline__ sym3 small_root(const small_strain &s) {
+  sym_power p{s.i1, -s.i2, s.i3};  // Z^3
+  float c2 = 0.5f + 0.5f * p.c2, c1 = 1.f + 0.5f * p.c1, c0 = 0.5f * p.c0;
+  const float v[6] = {0.375f, 0.375f, 0.3125f, 0.3125f, 0.2734375f, 0.2734375f};  // Z^4 ... Z^9
+#pragma unroll
+  for (int n = 0; n < 6; ++n) {
+    p.next(s.i1, s.i2, s.i3);
+    c2 += v[n] * p.c2, c1 += v[n] * p.c1, c0 += v[n] * p.c0;
+  }
+  return sym_poly(s.Z2, s.Z, c2, c1, c0);
+}
+
+__device__ __forceinline__ void store_sym(const sym3 &a, float *m) {
+  m[0] = a.xx, m[4] = a.yy, m[8] = a.zz;
+  m[1] = m[3] = a.xy;
+  m[2] = m[6] = a.xz;
+  m[5] = m[7] = a.yz;
+}
+
+// Fixed corotated at small strain: tau = V0 P F^T, with P F^T = 2 mu (b - sqrt(b)) + lambda J (J - 1) I
+// and b - sqrt(b) = E - (sqrt(b) - I).  False, with nothing written, where the strain is larger or F
+// a reflection (a NaN too).
+__device__ __forceinline__ bool constitutive_small(const material_dev &mat, const float *F, float *tau) {
+  const float J = det3(F);
+  small_strain s;
+  strain_of(F, s);
+  if (!(J > 0.f) || !(s.t2 <= kSmallRoot2)) return false;
+  const sym3 Y = small_root(s);
+  const float a = 2.f * mat.mu * mat.volume, b = mat.lambda * mat.volume * J * (J - 1.f);
+  store_sym(sym3{a * (s.E.xx - Y.xx) + b, a * (s.E.yy - Y.yy) + b, a * (s.E.zz - Y.zz) + b, a * (s.E.xy - Y.xy),
+                 a * (s.E.xz - Y.xz), a * (s.E.yz - Y.yz)},
+            tau);
+  return true;
+}
+
+// The constitutive update of G2P and G2P2G.  Fixed corotated takes the series where the strain is
+// small (kSeries; G2P commits no F for this model).  Drucker-Prager, whose committed F passes
+// through V every substep, and fixed corotated otherwise take svd3_columns; snow and whatever
+// these decline take svd3.
+// kWarp: every lane of the warp calls it together, and the Jacobi sweeps stop early.
+template <bool kWarp, bool kSeries>
+__device__ __forceinline__ void constitutive_update(const material_dev &mat, float *F, float &plastic, float *tau) {
+  bool done = false;
+  if (kSeries && mat.model == 0) {
+    done = constitutive_small(mat, F, tau);
+  } else if (mat.model != 2) {
+    float U[9], S[3], V[9];
+    done = svd3_columns<kWarp>(F, U, S, V);
+    if (done) constitutive_principal(mat, U, S, V, F, plastic, tau);
+  }
+  if (kWarp) {
+    const unsigned rest = __ballot_sync(0xffffffffu, !done);
+    if (!done) constitutive<true>(mat, F, plastic, tau, rest);
+  } else if (!done) {
+    constitutive<false>(mat, F, plastic, tau);
+  }
 }
 
 // ---------------------------------------------------------------- warp helpers

@@ -11,23 +11,28 @@ struct zsmpm_closure;
 
 namespace zsmpm {
 
-// One particle buffer set.  Vectors are float4 (x,y,z,m) / (vx,vy,vz,0).  3x3 matrices (C, A,
-// F) are stored in tiles of 32 particles: component k (column-major) of particle i at
+// One particle buffer set.  Positions are float4 (x,y,z,m).  3x3 matrices (C and F) are stored in tiles of 32 particles: component k (column-major) of particle i at
 // mat_at(k, i) = ((i / 32) * 9 + k) * 32 + i % 32, the layout of one 3x3 property of a
 // TileVector<float, 32>.  A warp's load of one component is 128 contiguous bytes, as with one
 // array per component, and its nine components of 32 particles are 1152 contiguous bytes: one
-// DRAM stream per matrix rather than nine (the G2P writes three matrices per particle).
+// DRAM stream per matrix rather than nine.
 // A matrix array holds 9 * mat_capacity(cap) floats.
 __host__ __device__ __forceinline__ size_t mat_at(int k, size_t i) {
   return ((i >> 5) * 9 + (size_t)k) * 32 + (i & 31);
 }
 __host__ __device__ __forceinline__ int64_t mat_capacity(int64_t cap) { return (cap + 31) & ~int64_t(31); }
 
+// What P2G reads beside x|m, the velocity and the affine momentum A = m C - (4 dt / dx^2) tau, is
+// kept per component d as float4 (v_d, A_d0, A_d1, A_d2), in tiles of 32 particles too: 16-byte
+// loads and stores, and 512 contiguous bytes for a warp's load of one component.
+__host__ __device__ __forceinline__ size_t row_at(int d, size_t i) {
+  return ((i >> 5) * 3 + (size_t)d) * 32 + (i & 31);
+}
+
 struct particle_buffers {
   float4 *xm = nullptr;
-  float4 *v = nullptr;
+  float4 *row = nullptr;  // 3 * mat_capacity(cap): (v_d, A_d0, A_d1, A_d2), consumed by P2G
   float *C = nullptr;
-  float *A = nullptr;  // affine momentum m C - (4 dt / dx^2) tau, consumed by P2G
   float *F = nullptr;
   float *plastic = nullptr;  // logJp (DP) or Jp (snow); null for fixed corotated
   int *id = nullptr;         // upload index
@@ -42,7 +47,7 @@ constexpr int kBatchMargin = 4;
 constexpr int kBatchMaxScenes = 1 << 16;
 
 // Device counters (int32), zeroed at the start of every substep except the status word, the
-// substep counter and the learned G2P's queue counters.
+// substep counter, the learned G2P's queue counters and the barrier's.
 enum counter_slot : int {
   kCtrParticleBlocks = 0,  // blocks inserted from particles (insertion indices [0, npb))
   kCtrEnlarged = 1,        // blocks inserted by the enlargement
@@ -64,7 +69,9 @@ enum counter_slot : int {
   kCtrDirty = 29,          // cells the incremental binning's movers arrived in (to be sorted by id)
   kCtrQueue = 30,          // projections the last learned G2P queued for the closure's network
   kCtrQueueSubstep = 31,   // the substep number of that G2P (the closure pass samples its audit by it)
-  kCtrCount = 32
+  kCtrBarrier = 32,        // k_prepare's grid barrier: arrivals, and CTAs that have left (both 0 between launches)
+  kCtrBarrierExit = 33,
+  kCtrCount = 34
 };
 enum work_slot : int {
   kWorkCellStart = 0,
@@ -104,6 +111,7 @@ struct scene_params {
   // incremental binning
   int mover_cap;                    // entries of the mover list
   int bin_full;                     // 1: this binning launch recounts every particle
+  int store_c;                      // 1: this G2P stores C, which no kernel of a substep reads
   int transfer;                     // kTransferApic (P2G / G2P) or kTransferCell (P2C2G / G2C2P)
 };
 
@@ -188,7 +196,7 @@ cudaError_t launch_p2c2g(scene_device &s, int part, cudaStream_t st);
 cudaError_t launch_grid_update(scene_device &s, cudaStream_t st);
 cudaError_t launch_g2p(scene_device &s, cudaStream_t st, bool closure_pass = true);
 cudaError_t launch_closure_pass(scene_device &s, cudaStream_t st);
-int kernels_per_substep();
+int kernels_per_substep(const scene_device &s);
 // the implicit system (ImplicitMPM.hpp) over node-major dof vectors [nb * 512 * 3]; a kernel
 // returns at once when `skip` (device, may be null) holds a nonzero value
 cudaError_t launch_g2p2g(scene_device &s, const float *v, float *f, long long ndofs, float dt, const int *skip,

@@ -8,6 +8,7 @@
 //   transfer    k_p2g, k_grid_update, k_g2p
 // Reference operators replaced: SparsityOp.hpp:41-112 (activation), SparsityOp.hpp:115-196
 // (binning), P2G.hpp:45-127, GridOp.hpp:54-164, G2P.hpp:43-84 (paths inside include/zensim).
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -82,11 +83,15 @@ __device__ int table_query(const scene_device &s, uint64_t key, int3 k) {
   return -1;
 }
 
+// x / dx + 1/2, whose floor is the index bucket (one rounding, written out so that every kernel that
+// asks for a particle's cell computes the same number)
+__device__ __forceinline__ float bucket_of(const scene_params &p, float x) { return fmaf(x, p.inv_dx, 0.5f); }
+
 // Stencil-origin cell and block of a position exactly as ComputeSparsity computes them
 // (SparsityOp.hpp:70-77): c = floor(x * (1/dx) + 0.5) - 2, block = floor_div(c, 8).
 // Returns false for NaN/Inf or positions beyond the packed key range.
 __device__ __forceinline__ bool cell_of(const scene_params &p, float4 x, int3 &c, int3 &b) {
-  const float fx = x.x * p.inv_dx + 0.5f, fy = x.y * p.inv_dx + 0.5f, fz = x.z * p.inv_dx + 0.5f;
+  const float fx = bucket_of(p, x.x), fy = bucket_of(p, x.y), fz = bucket_of(p, x.z);
   const float lim = (float)(kKeyLimit * 8);
   if (!(fabsf(fx) < lim && fabsf(fy) < lim && fabsf(fz) < lim)) return false;
   c = make_int3((int)floorf(fx) - 2, (int)floorf(fy) - 2, (int)floorf(fz) - 2);
@@ -94,12 +99,13 @@ __device__ __forceinline__ bool cell_of(const scene_params &p, float4 x, int3 &c
   return true;
 }
 
-// x / dx, as G2P and G2P2G compute the particle's position in cells (G2P.hpp:56-58,
-// G2P2G.hpp): a multiplication by 1/dx where dx is a power of two (the same number, since both
-// scale by a power of two exactly), else the correctly rounded division.  (In P2G the same
-// branch measured slower.)
+// x / dx for the particle's position in cells (P2G.hpp:62, G2P.hpp:56-58, G2P2G.hpp): the product
+// with the rounded reciprocal and one correction by the remainder (Markstein 1990), which is
+// the correctly rounded quotient but for rare last-place cases; where dx is a power of two the
+// product is exact and the correction zero.
 __device__ __forceinline__ float over_dx(const scene_params &p, float x) {
-  return p.dx_pow2 ? x * p.inv_dx : __fdiv_rn(x, p.dx);
+  const float q = x * p.inv_dx;
+  return fmaf(fmaf(-q, p.dx, x), p.inv_dx, q);
 }
 
 // Batched scenes: the slot of a scene, the slot coordinate of a key component (keys of a
@@ -224,7 +230,7 @@ cudaError_t device_scan(Load ld, const int *n_ptr, int *part, int *out, cudaStre
 
 // ----------------------------------------------------------------- activation
 // Resets the hash table (CleanSparsity, SparsityOp.hpp:41-55) and the per-substep counters.
-__global__ void __launch_bounds__(kThreads) k_begin(scene_device s) {
+__device__ __forceinline__ void do_begin(const scene_device &s) {
   const int T = s.prm.table_size;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < T; i += grid_threads()) {
     s.pk[i] = kEmptyKey;
@@ -240,7 +246,7 @@ __global__ void __launch_bounds__(kThreads) k_begin(scene_device s) {
     // the learned G2P's queue counters stay for a closure pass that runs beside this substep's
     // activation and binning (the learned G2P clears the queue before it fills it)
     if (t == kCtrStatus || t == kCtrMaskFrom || t == kCtrMaskBad || t == kCtrMovers || t == kCtrQueue ||
-        t == kCtrQueueSubstep)
+        t == kCtrQueueSubstep || t == kCtrBarrier || t == kCtrBarrierExit)
       return;
     if (t == kCtrUseMasks) {
       s.ctr[t] = s.ctr[kCtrMaskBad] == 0 ? s.ctr[kCtrMaskFrom] : 0;
@@ -262,9 +268,10 @@ __global__ void __launch_bounds__(kThreads) k_begin(scene_device s) {
     s.ctr[t] = v;
   }
 }
+__global__ void __launch_bounds__(kThreads) k_begin(scene_device s) { do_begin(s); }
 
 // ComputeSparsity (SparsityOp.hpp:58-86): one insert per distinct block key of a warp.
-__global__ void __launch_bounds__(kThreads) k_insert_particle_blocks(scene_device s) {
+__device__ __forceinline__ void do_insert_particle_blocks(const scene_device &s) {
   if (s.ctr[kCtrUseMasks] > 0) return;  // k_insert_moved_blocks inserts this substep's blocks
   const int lane = threadIdx.x & 31;
   const int n = s.prm.n;
@@ -321,12 +328,13 @@ __global__ void __launch_bounds__(kThreads) k_insert_particle_blocks(scene_devic
     atomicMax(&s.ctr[kCtrBoxHi + 2], hi.z);
   }
 }
+__global__ void __launch_bounds__(kThreads) k_insert_particle_blocks(scene_device s) { do_insert_particle_blocks(s); }
 
 // ComputeSparsity from the move masks the last G2P wrote: the blocks the particles of each
 // previous block ended in (the same set of keys as the particle pass finds, since G2P computes
 // each particle's block from the position it stores).  Runs instead of the particle pass
 // after a G2P in which no particle left its block's 3^3 neighbourhood.
-__global__ void __launch_bounds__(kThreads) k_insert_moved_blocks(scene_device s) {
+__device__ __forceinline__ void do_insert_moved_blocks(const scene_device &s) {
   const int nold = s.ctr[kCtrUseMasks];
   if (nold == 0) return;
   // the previous binning's block keys by their index then (k_assign_ranks renumbers blk_pk)
@@ -360,10 +368,11 @@ __global__ void __launch_bounds__(kThreads) k_insert_moved_blocks(scene_device s
     atomicMax(&s.ctr[kCtrBoxHi + 2], hi.z);
   }
 }
+__global__ void __launch_bounds__(kThreads) k_insert_moved_blocks(scene_device s) { do_insert_moved_blocks(s); }
 
 // EnlargeSparsity{lo=0, hi=2} (SparsityOp.hpp:88-112): the +{0,1}^3 neighbours of every
 // particle block, so that the 3x3x3 stencil of every particle lands in active blocks.
-__global__ void __launch_bounds__(kThreads) k_enlarge(scene_device s) {
+__device__ __forceinline__ void do_enlarge(const scene_device &s) {
   const int npb = min(s.ctr[kCtrParticleBlocks], s.prm.nb_cap);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npb * 7; t += grid_threads()) {
     const int i = t / 7, o = t % 7 + 1;
@@ -372,23 +381,21 @@ __global__ void __launch_bounds__(kThreads) k_enlarge(scene_device s) {
     table_insert(s, pack_key(nk.x, nk.y, nk.z), nk, &s.ctr[kCtrEnlarged], npb);
   }
 }
+__global__ void __launch_bounds__(kThreads) k_enlarge(scene_device s) { do_enlarge(s); }
 
-// Total block count, capacity checks and the dense bounding box of the bitmap that ranks
-// the blocks in ascending (bx, by, bz) order.
-__global__ void k_bitmap_prepare(scene_device s) {
-  if (threadIdx.x != 0) return;
-  s.ctr[kCtrMaskFrom] = 0;  // the masks are spent: the ranks below renumber the blocks
-  s.ctr[kCtrMaskBad] = 0;
+// Total block count, capacity checks and the words of the dense bitmap over the blocks' bounding
+// box, which ranks them in ascending (bx, by, bz) order.  `write`: the caller is the one thread
+// that records them.
+__device__ __forceinline__ void block_totals(const scene_device &s, bool write, int &blocks, int &words) {
   int nb = s.ctr[kCtrParticleBlocks] + s.ctr[kCtrEnlarged];
+  int st = 0;
   // HashTable.hpp:369 flags an insertion index >= T - 20, i.e. more than T - 20 blocks
-  if (nb > s.prm.table_size - 20) set_status(s.ctr, kStatusTableFull);
+  if (nb > s.prm.table_size - 20) st |= kStatusTableFull;
   if (nb > s.prm.nb_cap) {
-    set_status(s.ctr, kStatusCapacity);
+    st |= kStatusCapacity;
     nb = s.prm.nb_cap;
   }
-  s.ctr[kCtrBlocks] = nb;
-  *s.view_cnt = nb;
-  int words = 0;
+  words = 0;
   if (nb > 0) {
     const long long ex = (long long)s.ctr[kCtrBoxHi + 0] - s.ctr[kCtrBoxLo + 0] + 2;
     const long long ey = (long long)s.ctr[kCtrBoxHi + 1] - s.ctr[kCtrBoxLo + 1] + 2;
@@ -396,14 +403,25 @@ __global__ void k_bitmap_prepare(scene_device s) {
     const long long vol = ex * ey * ez;
     const long long w = (vol + 31) / 32;
     if (w > s.prm.bitmap_cap) {
-      set_status(s.ctr, kStatusBitmap);
-      s.ctr[kCtrBlocks] = 0;
-      *s.view_cnt = 0;
+      st |= kStatusBitmap;
+      nb = 0;
     } else {
       words = (int)w;
     }
   }
+  blocks = nb;
+  if (!write) return;
+  s.ctr[kCtrMaskFrom] = 0;  // the masks are spent: the ranks below renumber the blocks
+  s.ctr[kCtrMaskBad] = 0;
+  if (st) set_status(s.ctr, st);
+  s.ctr[kCtrBlocks] = nb;
+  *s.view_cnt = nb;
   s.ctr[kCtrWords] = words;
+}
+
+__global__ void k_bitmap_prepare(scene_device s) {
+  int nb, words;
+  if (threadIdx.x == 0) block_totals(s, true, nb, words);
 }
 
 __device__ __forceinline__ long long dense_id(const scene_device &s, int3 k) {
@@ -413,23 +431,24 @@ __device__ __forceinline__ long long dense_id(const scene_device &s, int3 k) {
          ((long long)k.z - s.ctr[kCtrBoxLo + 2]);
 }
 
-__global__ void __launch_bounds__(kThreads) k_bitmap_set(scene_device s) {
-  const int nb = s.ctr[kCtrWords] > 0 ? s.ctr[kCtrBlocks] : 0;
+__device__ __forceinline__ void do_bitmap_set(const scene_device &s, int nb) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += grid_threads()) {
     const long long d = dense_id(s, unpack_key(s.ins_pk[i]));
     atomicOr(&s.bitmap[d >> 5], 1u << (d & 31));
   }
 }
+__global__ void __launch_bounds__(kThreads) k_bitmap_set(scene_device s) {
+  do_bitmap_set(s, s.ctr[kCtrWords] > 0 ? s.ctr[kCtrBlocks] : 0);
+}
 
 // rank = number of active keys below this one; index == rank from here on
-__global__ void __launch_bounds__(kThreads) k_assign_ranks(scene_device s) {
-  const int nb = s.ctr[kCtrWords] > 0 ? s.ctr[kCtrBlocks] : 0;
+__device__ __forceinline__ void do_assign_ranks(const scene_device &s, int nb, const int *word_prefix) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += grid_threads()) {
     const uint64_t key = s.ins_pk[i];
     const int3 k = unpack_key(key);
     const long long d = dense_id(s, k);
     const uint32_t w = s.bitmap[d >> 5];
-    const int rank = s.word_prefix[d >> 5] + __popc(w & ((1u << (d & 31)) - 1u));
+    const int rank = word_prefix[d >> 5] + __popc(w & ((1u << (d & 31)) - 1u));
     s.tidx[s.ins_slot[i]] = rank;
     s.blk_pk[rank] = key;
     s.active_keys[3 * rank + 0] = k.x;
@@ -437,9 +456,12 @@ __global__ void __launch_bounds__(kThreads) k_assign_ranks(scene_device s) {
     s.active_keys[3 * rank + 2] = k.z;
   }
 }
+__global__ void __launch_bounds__(kThreads) k_assign_ranks(scene_device s) {
+  do_assign_ranks(s, s.ctr[kCtrWords] > 0 ? s.ctr[kCtrBlocks] : 0, s.word_prefix);
+}
 
 // neighbour table b + {0,1}^3 (index dx*4 + dy*2 + dz); clears the bitmap for next time
-__global__ void __launch_bounds__(kThreads) k_neighbors(scene_device s) {
+__device__ __forceinline__ void do_neighbors(const scene_device &s) {
   const int nb = s.ctr[kCtrBlocks];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nb * 8; t += grid_threads()) {
     const int b = t >> 3, o = t & 7;
@@ -450,6 +472,7 @@ __global__ void __launch_bounds__(kThreads) k_neighbors(scene_device s) {
   const int words = s.ctr[kCtrWords];
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += grid_threads()) s.bitmap[w] = 0u;
 }
+__global__ void __launch_bounds__(kThreads) k_neighbors(scene_device s) { do_neighbors(s); }
 
 // ----------------------------------------------------------------- binning
 // Per particle: its block index and stencil-origin cell; counts per cell (rank within the
@@ -458,7 +481,7 @@ __device__ __forceinline__ bool incremental_binning(const scene_device &s) {
   return s.ctr[kCtrIncBin] != 0 && !s.prm.bin_full;
 }
 
-__global__ void __launch_bounds__(kThreads) k_bin_count(scene_device s) {
+__device__ __forceinline__ void do_bin_count(const scene_device &s) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     s.ctr[kCtrOrderFront] = 0;  // k_cell_start fills work_order
     s.ctr[kCtrOrderBack] = 0;
@@ -468,7 +491,6 @@ __global__ void __launch_bounds__(kThreads) k_bin_count(scene_device s) {
     s.ctr[kCtrWork + kWorkFinalize] = 0;
     s.ctr[kCtrWork + kWorkP2G] = 0;
     s.ctr[kCtrWork + kWorkG2P] = 0;
-    s.ctr[kCtrDirty] = 0;
   }
   if (incremental_binning(s)) return;  // k_inc_stayers and k_inc_movers count this substep
   const int lane = threadIdx.x & 31;
@@ -525,6 +547,26 @@ __global__ void __launch_bounds__(kThreads) k_bin_count(scene_device s) {
    }
   }
 }
+__global__ void __launch_bounds__(kThreads) k_bin_count(scene_device s) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.ctr[kCtrDirty] = 0;
+  do_bin_count(s);
+}
+
+// The blocks that hold particles, in the order the per-block kernels take them: work_order holds
+// those of kBigBlock particles or more from the front and the others from the back.
+__device__ __forceinline__ int work_blocks(const scene_device &s) {
+  return s.ctr[kCtrOrderFront] + s.ctr[kCtrOrderBack];
+}
+__device__ __forceinline__ int work_block(const scene_device &s, int front, int nb, int w) {
+  return s.work_order[w < front ? w : nb - 1 - (w - front)];
+}
+
+// G2P's items: parts of a block's slots (each loads the block's velocity halo again, so a block is
+// split only where the blocks alone would leave SMs idle: measured with one split less or more,
+// 490 k particles 0.0645 / 0.0553 / 0.0557 ms, 3.7 M 0.245 / 0.236 / 0.26 ms.
+__device__ __forceinline__ int slot_parts(int nb, int ctas) {
+  return nb >= 4 * ctas ? 1 : nb * 2 >= 4 * ctas ? 2 : nb * 4 >= 4 * ctas ? 4 : 8;
+}
 
 // Persistent per-block CTA loop helper.
 __device__ __forceinline__ int grab_block(int *counter, int *s_b) {
@@ -551,15 +593,16 @@ __global__ void __launch_bounds__(512) k_cell_start(scene_device s) {
     s.cell_start[b * 512 + threadIdx.x] = s.block_start[b] + ex;
     // the per-block kernels take the big blocks first, so that they end on small ones
     if (threadIdx.x == 0) {
+      s.bmask[b] = 0u;  // (G2P's items add to it)
       if (total >= kBigBlock)
         s.work_order[atomicAdd(&s.ctr[kCtrOrderFront], 1)] = b;
-      else
+      else if (total > 0)
         s.work_order[nb - 1 - atomicAdd(&s.ctr[kCtrOrderBack], 1)] = b;
     }
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_bin_scatter(scene_device s) {
+__device__ __forceinline__ void do_bin_scatter(const scene_device &s) {
   if (incremental_binning(s)) return;
   const int n = s.prm.n;
   const int stride = grid_threads();
@@ -579,6 +622,7 @@ __global__ void __launch_bounds__(kThreads) k_bin_scatter(scene_device s) {
       if (k[u] != 0xffffffffu) s.tmp[cs[u] + r[u]] = i0 + u * stride;
   }
 }
+__global__ void __launch_bounds__(kThreads) k_bin_scatter(scene_device s) { do_bin_scatter(s); }
 
 // Orders the list of one cell (indices into cur) by upload id, from `in` into `out` (which may
 // be the same array).  Lists of up to 12 entries are sorted in registers (every index known at
@@ -690,7 +734,10 @@ __device__ __forceinline__ int2 prev_cell_range(const scene_device &s, int j) {
   return make_int2(cs, ce);
 }
 
-__global__ void __launch_bounds__(kThreads) k_inc_stayers(scene_device s) {
+// kFused: within the fused kernel, where the movers are counted in the same phase (the counts are
+// added, not stored) and the new block indices are found here
+template <bool kFused>
+__device__ __forceinline__ void do_inc_stayers(const scene_device &s) {
   if (!incremental_binning(s)) return;
   const int nold = s.ctr[kCtrUseMasks], nb = s.ctr[kCtrBlocks];
   const long long cells = (long long)nold * 512;  // a warp covers 32 cells of one block
@@ -699,6 +746,15 @@ __global__ void __launch_bounds__(kThreads) k_inc_stayers(scene_device s) {
     const long long j = j0 + threadIdx.x;
     const bool in = j < cells;
     int stay = 0, nbi = -1;
+    if (kFused && j0 + (threadIdx.x & ~31) < cells) {  // (a warp's cells are of one block)
+      const int b = (int)((j0 + (threadIdx.x & ~31)) >> 9);
+      if (lane == 0) {
+        const uint64_t key = s.old_pk[b];
+        nbi = table_query(s, key, unpack_key(key));
+        if (((j0 + threadIdx.x) & 511) == 0) s.new_of_old[b] = nbi;
+      }
+      nbi = __shfl_sync(kFull, nbi, 0);
+    }
     if (in) {
       const int2 r = prev_cell_range(s, (int)j);
       int slot = r.x;
@@ -707,19 +763,23 @@ __global__ void __launch_bounds__(kThreads) k_inc_stayers(scene_device s) {
         stay += (a == 0) + (b1 == 0) + (c == 0) + (d == 0);
       }
       for (; slot < r.y; ++slot) stay += s.moved[slot] == 0;
-      nbi = s.new_of_old[(int)(j >> 9)];
+      if (!kFused) nbi = s.new_of_old[(int)(j >> 9)];
       if (stay > 0xffff) set_status(s.ctr, kStatusCapacity);  // shares its word with the arrivals
-      if (nbi >= 0 && nbi < nb)
-        s.cell_count[nbi * 512 + (int)(j & 511)] = stay;
-      else if (stay > 0)
+      if (nbi >= 0 && nbi < nb) {
+        if (!kFused)
+          s.cell_count[nbi * 512 + (int)(j & 511)] = stay;
+        else if (stay > 0)
+          atomicAdd(&s.cell_count[nbi * 512 + (int)(j & 511)], stay);
+      } else if (stay > 0)
         set_status(s.ctr, kStatusMissingBlock);
     }
     const int wsum = __reduce_add_sync(kFull, stay);
     if (lane == 0 && wsum > 0 && nbi >= 0 && nbi < nb) atomicAdd(&s.block_count[nbi], wsum);
   }
 }
+__global__ void __launch_bounds__(kThreads) k_inc_stayers(scene_device s) { do_inc_stayers<false>(s); }
 
-__global__ void __launch_bounds__(kThreads) k_inc_movers(scene_device s) {
+__device__ __forceinline__ void do_inc_movers(const scene_device &s) {
   if (!incremental_binning(s)) return;
   const int nmov = min(s.ctr[kCtrMovers], s.prm.mover_cap);
   const int nb = s.ctr[kCtrBlocks];
@@ -743,8 +803,9 @@ __global__ void __launch_bounds__(kThreads) k_inc_movers(scene_device s) {
     s.mover_pos[k] = pos;
   }
 }
+__global__ void __launch_bounds__(kThreads) k_inc_movers(scene_device s) { do_inc_movers(s); }
 
-__global__ void __launch_bounds__(kThreads) k_inc_place_stayers(scene_device s) {
+__device__ __forceinline__ void do_inc_place_stayers(const scene_device &s) {
   if (!incremental_binning(s)) return;
   const int nold = s.ctr[kCtrUseMasks], nb = s.ctr[kCtrBlocks];
   const long long cells = (long long)nold * 512;
@@ -764,8 +825,9 @@ __global__ void __launch_bounds__(kThreads) k_inc_place_stayers(scene_device s) 
     }
   }
 }
+__global__ void __launch_bounds__(kThreads) k_inc_place_stayers(scene_device s) { do_inc_place_stayers(s); }
 
-__global__ void __launch_bounds__(kThreads) k_inc_place_movers(scene_device s) {
+__device__ __forceinline__ void do_inc_place_movers(const scene_device &s) {
   if (!incremental_binning(s)) return;
   const int nmov = min(s.ctr[kCtrMovers], s.prm.mover_cap);
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nmov; k += grid_threads()) {
@@ -774,6 +836,7 @@ __global__ void __launch_bounds__(kThreads) k_inc_place_movers(scene_device s) {
     s.src[s.cell_start[pos.x] + (s.cell_count[pos.x] & 0xffff) + pos.y] = s.movers[k];
   }
 }
+__global__ void __launch_bounds__(kThreads) k_inc_place_movers(scene_device s) { do_inc_place_movers(s); }
 
 // the cells that received movers, in upload-id order (stayers and arrivals merged)
 __global__ void __launch_bounds__(kThreads) k_inc_sort(scene_device s) {
@@ -805,432 +868,376 @@ __global__ void __launch_bounds__(kThreads) k_inc_finalize(scene_device s) {
 }
 
 // ----------------------------------------------------------------- P2G
-// One CTA per block (persistent).  The block's 512 cells are processed in chunks of 64:
-//  1. the CTA gathers the chunk's particles, two per thread with their loads issued together,
-//     and stages, per particle, its 3x3 B-spline weights, m and the affine terms (q, A dx) in
-//     shared memory as six float4 fields laid out [field][rank][cell], rows padded by one
-//     float4: lanes reading one rank of consecutive cells read 512 contiguous bytes, and the
-//     ranks of one cell, which consecutive lanes write, start 4 banks apart;
-//  2. one thread per (cell, channel) sums the cell's particles into 27 registers -- all
-//     particles of a cell share the same 27 stencil nodes -- and adds them to a halo of the
-//     grid in shared memory.
-// Ranks are staged R at a time: a chunk with a cell of more particles runs phases 1-2 again for
-// the next ranks (a round), so that no particle needs the slow per-node path for lack of
-// staging room and the staging stays small enough for several CTAs per SM.
-// The halo holds the nodes the block's particles reach: a particle binned in cell c of the
-// block has its stencil origin at c + 1 (SparsityOp.hpp:72-77 against P2G.hpp:62-66), so its
-// nodes lie in [8b + 1, 8b + 11) per axis; the halo spans exactly that in x and y and
-// [8b, 8b + 12) in z, so that the flush moves whole 16-byte quads of the neighbour blocks.
-// Grid channels: m and p = sum W (m v + A (x_i - x_p)), the reference's mv + rhs
-// (P2G.hpp:108-125) with A = m C - (4 dt/dx^2) tau precomputed by G2P.
-// The staging depth is a tile choice of the autotuner: R particles per cell are staged per
-// round, with the register budget cut for the CTAs per SM that R's shared memory allows --
-// 8 ranks (55 KB) for 4 CTAs per SM, 12 (72 KB, the default) for 3, 16 (88 KB) for 2.
-// ZSMPM_P2G_STAGE_F = 1 (compile-time) stages the particle's fractional position in the cell
-// instead of its nine weights (phase 2 recomputes them: more arithmetic, a third less shared
-// memory).
-#ifndef ZSMPM_P2G_STAGE_F
-#define ZSMPM_P2G_STAGE_F 1
-#endif
-constexpr int kP2GChunk = 64;     // cells per chunk
-constexpr int kP2GRanksDefault = 12;  // particles per cell staged per round, unless tuned
-constexpr bool kP2GStageF = ZSMPM_P2G_STAGE_F != 0;
-constexpr int kP2GRow = kP2GChunk + 1;  // padded row of float4: rank r of cell c at bank 4 (r + c) % 32
-constexpr int kP2GThreads = 256;  // 4 channels x 64 cells
-constexpr int kP2GMap = 1024;     // slots of a chunk mapped to their cell (more: binary search)
-constexpr int kP2GHx = 10, kP2GHy = 10, kP2GHz = 12;  // halo extents (x, y from 8b + 1; z from 8b)
-constexpr int kP2GHaloNodes = kP2GHx * kP2GHy * kP2GHz;
+// Work items are (block, range of x planes); a CTA of four warps takes one at a time.  Warp w
+// owns the 16 cells y in {2w, 2w + 1}, z in 0..7 of every plane, two lanes per cell: one sums
+// the channels (m, p_x), the other (p_y, p_z), as packed pairs (fma.rn.f32x2).  All particles of
+// a cell share its 27 stencil nodes, so a lane keeps 27 pair sums in registers; it walks the
+// cells of its (y, z) column along x and the sums slide with it: after each plane the nine
+// leading nodes are complete for this column and go to the node plane in shared memory (shared
+// atomics), and the other eighteen carry over.  A cell thus adds 9 nodes instead of 27, and the
+// node plane, two deep, replaces a halo of the whole block.  Grid channels: m and
+// p = sum W (m v + A (x_i - x_p)), the reference's mv + rhs (P2G.hpp:108-125) with
+// A = m C - (4 dt/dx^2) tau precomputed by G2P.
+//
+// The particles come through a ring of S windows per warp: a window holds four ranks of the
+// warp's 16 cells, 64 bytes a particle (x|m and the three rows v_d, A_d0..2), fetched with
+// 16-byte cp.async in the order of the slot map, so that neighbouring lanes read neighbouring
+// particles.  The slot-map entries are loaded one window ahead of the copies.  Warps depend on
+// each other only in the node planes (one barrier per plane).
+//
+// A particle binned in cell c of the block has its stencil origin at c + 1 (SparsityOp.hpp:72-77
+// against P2G.hpp:62-66).  Where rounding puts x / dx on the other side of a cell boundary
+// (dx not a power of two) its weights are evaluated at f just outside [0.5, 1.5): the quadratic
+// B-spline is C1 there, so the difference is of second order in that rounding.
+//
+// What bounds it: instruction issue, about 300 thread instructions a particle (27 nodes x 4
+// channels x 2 operations in pairs, 108; weights, staging and emission the rest); the 68 bytes a
+// particle are 0.31 ms of a 30 M-particle launch.
+constexpr int kP2GThreads = 128;
+constexpr int kP2GRanksDefault = 8;  // ranks in flight per cell unless tuned: windows of 4, 2 deep
+constexpr int kP2GWin = 4;            // ranks per window
+constexpr int kP2GRow = 17;           // float4 row of 16 cells, padded (copies of one cell's ranks hit other banks)
+constexpr int kP2GField = kP2GWin * kP2GRow;  // float4 of one field of a window
+constexpr int kP2GStage = 4 * kP2GField;      // float4 of a window
+constexpr int kP2GUnit = kP2GField + kP2GRow; // the mass channel's rows, read one rank past the end
+// A warp's share of a node plane: [channel][4 y][12 z] floats (z from 8b; rows 2w .. 2w + 3 of the
+// block's ten), the channels padded so that a warp's stores of two channels fall on distinct banks.
+// Node planes are kept four deep (two barriers apart).
+constexpr int kP2GPlaneRow = 12, kP2GPlaneCh = 4 * kP2GPlaneRow + 4, kP2GPlane = 4 * kP2GPlaneCh;
 
-struct p2g_particle {
-  float m, w[3][3], f[3], q[3], ax[3], ay[3], az[3];
-  int hb[3];  // stencil origin relative to the block's first cell 8b (1..8 when binned in it)
-};
-
-// quadratic B-spline weights of the nodes 0, 1, 2 of a stencil at fractional position f
-// (InterpolationKernel.hpp:93-130)
-__device__ __forceinline__ void bspline_weights(float f, float *w) {
-  w[0] = 0.5f * (1.5f - f) * (1.5f - f);
-  const float f1 = f - 1.f;
-  w[1] = 0.75f - f1 * f1;
-  const float f2 = 0.5f + f1;
-  w[2] = 0.5f * f2 * f2;
+constexpr size_t p2g_smem_bytes(int ranks) {
+  return sizeof(float4) * ((size_t)4 * (ranks / kP2GWin) * kP2GStage + kP2GUnit) + sizeof(float) * 4 * 4 * kP2GPlane +
+         sizeof(int) * 2 * 528;
 }
 
-// The node weights of the cell-centric pair (P2C2GTransfer): a particle's tent weights to the
-// centers of its two cells per axis, 1/2 - fx and 1/2 + fx with fx = x/dx - floor(x/dx + 1/2),
+// cp.async (sm_80 and later): copies that land in shared memory while the warp computes
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(a), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { cp_async_wait<0>(); }
+
+__device__ __forceinline__ float2 shfl_up2(float2 a, int d) {
+  return make_float2(__shfl_up_sync(kFull, a.x, d), __shfl_up_sync(kFull, a.y, d));
+}
+__device__ __forceinline__ float2 shfl_down2(float2 a, int d) {
+  return make_float2(__shfl_down_sync(kFull, a.x, d), __shfl_down_sync(kFull, a.y, d));
+}
+__device__ __forceinline__ float2 shfl_xor2(float2 a, int d) {
+  return make_float2(__shfl_xor_sync(kFull, a.x, d), __shfl_xor_sync(kFull, a.y, d));
+}
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+
+// Twice the quadratic B-spline weights (InterpolationKernel.hpp:93-130) of the nodes 0, 1, 2 of a
+// stencil for nh = 1 - f, the distance from the particle to the middle node in cells, in both
+// halves of a pair.  (The factor two drops the halvings; it is a power of two, so the products
+// of three such weights with data scaled by 1/8 round as the plain ones do.)
+__device__ __forceinline__ void bspline_weights2(float2 nh, float2 *w) {
+  const float2 t = add2(nh, dup2(0.5f));
+  w[0] = mul2(t, t);
+  w[1] = fma2(mul2(nh, dup2(-2.f)), nh, dup2(1.5f));
+  const float2 g = fma2(nh, dup2(-1.f), dup2(0.5f));
+  w[2] = mul2(g, g);
+}
+
+// Twice the node weights of the cell-centric pair (P2C2GTransfer): a particle's tent weights to
+// the centers of its two cells per axis, 1/2 - fx and 1/2 + fx with fx = x/dx - floor(x/dx + 1/2),
 // each passed half to either corner, over the nodes base .. base + 2 (base = floor(x/dx + 1/2)
-// - 1, f = x/dx - base = fx + 1).
-__device__ __forceinline__ void cell_weights(float f, float *w) {
-  w[0] = 0.75f - 0.5f * f;
-  w[1] = 0.5f;
-  w[2] = 0.5f * f - 0.25f;
+// - 1, fx = -nh).
+__device__ __forceinline__ void cell_weights2(float2 nh, float2 *w) {
+  w[0] = add2(nh, dup2(0.5f));
+  w[1] = dup2(1.f);
+  w[2] = fma2(nh, dup2(-1.f), dup2(0.5f));
 }
 
-struct p2g_raw {
-  float4 xm, v;
-  float A[9];
-};
-
-__device__ __forceinline__ void p2g_load(const scene_device &s, const float *affine, int i, p2g_raw &r) {
-  r.xm = s.cur.xm[i];
-  r.v = s.cur.v[i];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) r.A[k] = affine[mat_at(k, i)];
+// Parts a block's eight x planes are split into (work items of 8 / parts planes each): one where
+// the blocks alone fill the chip several times over, more where they do not (a block's particles
+// would otherwise be one CTA's serial work while other SMs idle).
+__device__ __forceinline__ int plane_parts(int nb, int ctas) {
+  return nb >= 4 * ctas ? 1 : nb * 2 >= 4 * ctas ? 2 : nb * 4 >= 4 * ctas ? 4 : 8;
 }
 
-// kCell: the cell-centric pair's weights and stencil origin; with_mass = false leaves the mass
-// and the m v term out (P2C2GTransferForce)
-template <bool kCell>
-__device__ __forceinline__ void p2g_prepare(const scene_params &p, const p2g_raw &r, int ox, int oy, int oz,
-                                            p2g_particle &pp, bool with_mass) {
-  // APIC: x / dx as P2G.hpp:62 divides (a multiplication when dx is a power of two, the same
-  // number).  The cell pair: the index bucket floor(x * (1/dx) + 1/2) as the binning keys it.
-  float X[3];
-  if (kCell) {
-    X[0] = r.xm.x * p.inv_dx, X[1] = r.xm.y * p.inv_dx, X[2] = r.xm.z * p.inv_dx;
-  } else {
-    X[0] = over_dx(p, r.xm.x), X[1] = over_dx(p, r.xm.y), X[2] = over_dx(p, r.xm.z);
-  }
-  float lp[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const float base = kCell ? floorf(X[d] + 0.5f) - 1.f : floorf(X[d] - 0.5f);
-    const float f = X[d] - base;
-    pp.hb[d] = (int)base - (d == 0 ? ox : d == 1 ? oy : oz);
-    pp.f[d] = f;
-    if (kCell)
-      cell_weights(f, pp.w[d]);
-    else
-      bspline_weights(f, pp.w[d]);
-    lp[d] = f * p.dx;
-  }
-  pp.m = with_mass ? r.xm.w : 0.f;
-  const float vel[3] = {r.v.x, r.v.y, r.v.z};
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    pp.q[d] = pp.m * vel[d] - (r.A[d] * lp[0] + r.A[3 + d] * lp[1] + r.A[6 + d] * lp[2]);
-    pp.ax[d] = r.A[d] * p.dx;
-    pp.ay[d] = r.A[3 + d] * p.dx;
-    pp.az[d] = r.A[6 + d] * p.dx;
-  }
-}
+// kCell: P2C2GTransfer of the cell-centric pair (below) with the pair's node weights and affine
+// term; `rows` holds v and the affine term (A = m C - (4 dt/dx^2) tau for APIC), with_mass = 0
+// leaves the mass channel and the m v term out.  S windows in the ring (the staging depth of the
+// tuner: 8, 12 or 16 ranks).
+template <bool kCell, int S>
+__global__ void __launch_bounds__(kP2GThreads, 4) k_p2g(scene_device s, const float4 *rows, int with_mass) {
+  extern __shared__ __align__(16) float4 p2g_smem[];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  float4 *const ring = p2g_smem + w * S * kP2GStage;
+  float4 *const unit = p2g_smem + 4 * S * kP2GStage;  // (1, 0, 0, 0): the mass channel's row
+  float *const plane = reinterpret_cast<float *>(unit + kP2GUnit);
+  // per item parity: the block's 512 cell starts and its end, its neighbours and its key
+  int *const meta = reinterpret_cast<int *>(plane + 16 * kP2GPlane);
+  constexpr int kMeta = 528, kMetaEnd = 512, kMetaKey = 514, kMetaNbr = 516;
+  __shared__ int s_item[2];
+  __shared__ unsigned char s_hot[4][4];  // [node plane][warp]: the warp added to it
+  const scene_params &prm = s.prm;
+  const int nb = s.ctr[kCtrBlocks], front = s.ctr[kCtrOrderFront], nwork = work_blocks(s);
+  const int parts = plane_parts(nwork, gridDim.x), nx = 8 / parts, items = nwork * parts;
+  int *const counter = &s.ctr[kCtrWork + kWorkP2G];
+  for (int q = t; q < kP2GUnit; q += kP2GThreads) unit[q] = make_float4(1.f, 0.f, 0.f, 0.f);
+  for (int q = t; q < 16 * kP2GPlane; q += kP2GThreads) plane[q] = 0.f;
 
-// Every node of one particle by itself: shared atomics into the halo when its stencil lies in
-// it, else global atomics into the grid blocks b + {0,1}^3 (a stencil origin that rounding
-// put one cell off the binned cell, possible when dx is not a power of two).
-__device__ __forceinline__ void p2g_direct(const scene_device &s, float *sh, const p2g_particle &pp, int b) {
-  const int hx = pp.hb[0] - 1, hy = pp.hb[1] - 1, hz = pp.hb[2];
-  const bool in_halo = hx >= 0 && hx <= kP2GHx - 3 && hy >= 0 && hy <= kP2GHy - 3 && hz >= 0 && hz <= kP2GHz - 3;
-  const bool in_reach = pp.hb[0] >= 0 && pp.hb[0] <= 13 && pp.hb[1] >= 0 && pp.hb[1] <= 13 && pp.hb[2] >= 0 &&
-                        pp.hb[2] <= 13;
-  if (!in_halo && !in_reach) {
-    set_status(s.ctr, kStatusMissingBlock);
-    return;
+  auto fetch_meta = [&](int *m, int b) {
+    cp_async16(m + 4 * t, s.cell_start + (size_t)b * 512 + 4 * t);
+    if (t == 0) cp_async4(m + kMetaEnd, s.block_start + b + 1);
+    if (t < 2) {
+      cp_async16(m + kMetaNbr + 4 * t, s.nbr + (size_t)b * 8 + 4 * t);
+      cp_async4(m + kMetaKey + t, reinterpret_cast<const int *>(s.blk_pk + b) + t);
+    }
+    cp_async_commit();
+  };
+
+  int ahead = 0;  // thread 0: the item after next
+  if (t == 0) {
+    s_item[0] = atomicAdd(counter, 1);
+    ahead = atomicAdd(counter, 1);
   }
-  for (int ii = 0; ii < 3; ++ii)
-    for (int jj = 0; jj < 3; ++jj)
-      for (int kk = 0; kk < 3; ++kk) {
-        const float W = pp.w[0][ii] * pp.w[1][jj] * pp.w[2][kk];
-        float v[4];
-        v[0] = W * pp.m;
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          v[1 + d] = W * (pp.q[d] + (float)ii * pp.ax[d] + (float)jj * pp.ay[d] + (float)kk * pp.az[d]);
-        if (in_halo) {
-          const int h = ((hx + ii) * kP2GHy + (hy + jj)) * kP2GHz + hz + kk;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) atomicAdd(&sh[c * kP2GHaloNodes + h], v[c]);
-        } else {
-          const int X = pp.hb[0] + ii, Y = pp.hb[1] + jj, Z = pp.hb[2] + kk;  // cells from 8b
-          if (X >= 16 || Y >= 16 || Z >= 16) {
-            set_status(s.ctr, kStatusMissingBlock);
-            continue;
-          }
-          const int tb = s.nbr[b * 8 + ((X >> 3) << 2) + ((Y >> 3) << 1) + (Z >> 3)];
-          if (tb < 0) {
-            set_status(s.ctr, kStatusMissingBlock);
-            continue;
-          }
-          const int cell = ((X & 7) << 6) | ((Y & 7) << 3) | (Z & 7);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) atomicAdd(&s.grid[((size_t)tb * kGridChannels + c) * 512 + cell], v[c]);
+  __syncthreads();
+  int item = s_item[0];
+  if (item < items) fetch_meta(meta, work_block(s, front, nb, item / parts));
+  // the lane's cell column, channels and constants
+  const int cell16 = lane & 15, pair = lane >> 4;
+  const int ly = 2 * w + (cell16 >> 3), lz = cell16 & 7;
+  // the weights below are twice the stencil's, so the data carry 1/8
+  const float2 dx8 = dup2(0.125f * prm.dx);
+  const float mscale = with_mass ? 0.125f : 0.f;
+  // where the lane stores the node sums it ends up with: row 2 (ly & 1), node z = lz + 1 from 8b
+  float *const emit0 = plane + w * kP2GPlane + 2 * pair * kP2GPlaneCh + 2 * (ly & 1) * kP2GPlaneRow + lz + 1;
+  // the copies of a window: ranks lane & 3 of the cells lane >> 2 and (lane >> 2) + 8
+  const int cp_cell = lane >> 2, cp_rank = lane & 3;
+  float4 *const cp_dst = ring + cp_rank * kP2GRow + cp_cell;
+
+  for (int par = 0; item < items; par ^= 1) {
+    if (t == 0) {
+      s_item[par ^ 1] = ahead;
+      ahead = atomicAdd(counter, 1);
+    }
+    cp_async_wait_all();
+    __syncthreads();  // this item's starts are in place; the last item is done with the other set
+    const int *const cs = meta + par * kMeta;
+    const int next = s_item[par ^ 1];
+    const int next_b = next < items ? work_block(s, front, nb, next / parts) : -1;
+    const int x0 = item % parts * nx, x1 = x0 + nx;
+    if (cs[x0 * 64] == cs[x1 * 64]) {  // (cs[512] is the block's end)
+      if (next_b >= 0) fetch_meta(meta + (par ^ 1) * kMeta, next_b);
+      item = next;
+      continue;
+    }
+    const uint64_t key = (uint64_t)(uint32_t)cs[kMetaKey] | ((uint64_t)(uint32_t)cs[kMetaKey + 1] << 32);
+    const int3 bk = local_block(prm, unpack_key(key));
+    // the stencils' middle nodes
+    const float by = (float)(bk.y * 8 + ly + 2), bz = (float)(bk.z * 8 + lz + 2);
+
+    // ---- the ring's producers: slot-map entries (one window ahead), then the copies
+    int lx = x0 - 1, lrank = 0, lmax = 0;  // the window whose slot-map entries are loaded next
+    int src0 = -1, src1 = -1;
+    int fill = 0;  // ring stage the next copies go to
+    const int *const mycells = cs + 16 * w;
+    auto load_src = [&]() {
+      while (lrank >= lmax && lx < x1) {  // next plane with particles in the warp's cells
+        lrank = 0;
+        lmax = 0;
+        if (++lx < x1) {
+          const int c = lx * 64 + cell16;
+          lmax = __reduce_max_sync(kFull, mycells[c + 1] - mycells[c]);
         }
       }
-}
-
-// float4 fields: w00 w01 w02 w10 | w11 w12 w20 w21 | w22 m | (q ax ay az) x 3, or with the
-// fractional position: fx fy fz m | (q ax ay az) x 3
-constexpr int kP2GVec = kP2GStageF ? 4 : 6;
-constexpr int kP2GQ = kP2GVec - 3;  // first momentum field
-constexpr size_t p2g_smem_bytes(int ranks) {
-  return sizeof(float) * kGridChannels * kP2GHaloNodes + sizeof(float4) * kP2GVec * ranks * kP2GRow +
-         sizeof(int) * 2 * (kP2GChunk + 1) + sizeof(int) * 4 + sizeof(unsigned char) * 2 * kP2GMap;
-}
-
-// the weights and the mass of staged rank r of cell cl
-template <bool kCell, int R>
-__device__ __forceinline__ void staged_weights(const float4 (*stg)[R][kP2GRow], int r, int cl, float (&w)[3][3],
-                                               float &m) {
-  if (kP2GStageF) {
-    const float4 fm = stg[0][r][cl];
-    if (kCell) {
-      cell_weights(fm.x, w[0]);
-      cell_weights(fm.y, w[1]);
-      cell_weights(fm.z, w[2]);
-    } else {
-      bspline_weights(fm.x, w[0]);
-      bspline_weights(fm.y, w[1]);
-      bspline_weights(fm.z, w[2]);
-    }
-    m = fm.w;
-  } else {
-    const float4 wa = stg[0][r][cl], wb = stg[1][r][cl], wc = stg[2][r][cl];
-    w[0][0] = wa.x, w[0][1] = wa.y, w[0][2] = wa.z;
-    w[1][0] = wa.w, w[1][1] = wb.x, w[1][2] = wb.y;
-    w[2][0] = wb.z, w[2][1] = wb.w, w[2][2] = wc.x;
-    m = wc.y;
-  }
-}
-
-// kCell: P2C2GTransfer of the cell-centric pair (below) with the pair's node weights and
-// affine term; `affine` is the affine term (A = m C - (4 dt/dx^2) tau for APIC), with_mass = 0
-// leaves the mass channel and the m v term out.  R staged ranks per round, registers cut for
-// MinCtas CTAs per SM.
-template <bool kCell, int R, int MinCtas>
-__global__ void __launch_bounds__(kP2GThreads, MinCtas) k_p2g(scene_device s, const float *affine, int with_mass) {
-  extern __shared__ __align__(16) float p2g_smem[];
-  float *sh = p2g_smem;
-  auto stg = reinterpret_cast<float4(*)[R][kP2GRow]>(p2g_smem + kGridChannels * kP2GHaloNodes);
-  int *s_cs = reinterpret_cast<int *>(p2g_smem + kGridChannels * kP2GHaloNodes +
-                                      4 * kP2GVec * R * kP2GRow);
-  int *const s_wmax = s_cs + 2 * (kP2GChunk + 1);  // per chunk parity: the largest cell count of each half
-  unsigned char *const s_map0 = reinterpret_cast<unsigned char *>(s_wmax + 4);
-  __shared__ int s_b;
-  const int nb = s.ctr[kCtrBlocks];
-  const int t = threadIdx.x;
-  const int my_cell = t & (kP2GChunk - 1), my_ch = t >> 6;
-  // the halo starts zeroed; each block's flush zeroes the quads it sends, so the next block
-  // finds it zeroed again (the first barrier of grab_block orders both)
-  for (int q = t; q < kGridChannels * kP2GHaloNodes; q += blockDim.x) sh[q] = 0.f;
-  for (;;) {
-    const int w = grab_block(&s.ctr[kCtrWork + kWorkP2G], &s_b);
-    if (w >= nb) break;
-    const int b = s.work_order[w];
-    const int start = s.block_start[b], end = s.block_start[b + 1];
-    if (start == end) continue;
-    const int3 bk = local_block(s.prm, unpack_key(s.blk_pk[b]));
-    const int ox = bk.x * 8, oy = bk.y * 8, oz = bk.z * 8;
-    int *const s_cs0 = s_cs;
-    // cell starts of chunk k in s_cs0 + (k & 1) * (kP2GChunk + 1), its slot -> cell map in
-    // s_map0 + (k & 1) * kP2GMap and its largest cell count in s_wmax[2 (k & 1) ..]; the next
-    // chunk's are filled during this chunk's last phase 2, so a round needs two barriers
-    auto fill = [&](int chunk_to_fill) {
-      if (t <= kP2GChunk) {
-        const int c = chunk_to_fill * kP2GChunk + t;
-        s_cs0[(chunk_to_fill & 1) * (kP2GChunk + 1) + t] = c < 512 ? s.cell_start[b * 512 + c] : end;
-      }
-      if (t < kP2GChunk) {
-        const int c = chunk_to_fill * kP2GChunk + t;
-        const int cs = s.cell_start[b * 512 + c];
-        const int ce = c + 1 < 512 ? s.cell_start[b * 512 + c + 1] : end;
-        const int base = s.cell_start[b * 512 + chunk_to_fill * kP2GChunk];
-        unsigned char *m = s_map0 + (chunk_to_fill & 1) * kP2GMap;
-        for (int q = cs - base; q < ce - base && q < kP2GMap; ++q) m[q] = (unsigned char)t;
-        const int wmax = __reduce_max_sync(kFull, ce - cs);
-        if ((t & 31) == 0) s_wmax[2 * (chunk_to_fill & 1) + (t >> 5)] = wmax;
+      src0 = src1 = -1;
+      if (lx < x1) {
+        const int c = lx * 64 + cp_cell;
+        const int a = mycells[c] + lrank + cp_rank, b = mycells[c + 8] + lrank + cp_rank;
+        if (a < mycells[c + 1]) src0 = s.src[a];
+        if (b < mycells[c + 9]) src1 = s.src[b];
+        lrank += kP2GWin;
       }
     };
-    fill(0);
-    // the shallow (8-rank) staging, which the tuner picks for sparse cells: the slot-map entries
-    // of this thread's first two slots of the next chunk are loaded during the current chunk's
-    // last sums, so that the next phase 1 waits for one load instead of two (-1: not loaded).
-    // At 8 ranks this measured 1.035 against 1.067 ms on the 16 M snow scene; at 12 ranks it
-    // was slower.
-    constexpr bool kPrefetchSrc = R == 8;
-    int pre1 = -1, pre2 = -1;
-    for (int chunk = 0; chunk < 512 / kP2GChunk; ++chunk) {
-      const int cell0 = chunk * kP2GChunk;
-      const int par = chunk & 1;
-      int *s_cs = s_cs0 + par * (kP2GChunk + 1);
-      const unsigned char *s_map = s_map0 + par * kP2GMap;
-      for (int round = 0;; ++round) {
-        __syncthreads();  // previous staging consumed, this chunk's starts loaded, halo zeroed
-        const int maxc = max(s_wmax[2 * par], s_wmax[2 * par + 1]);
-        const int rlo = round * R;
-        const bool last = rlo + R >= maxc;
-        // ---- phase 1: consecutive threads take consecutive slots (coalesced gathers); the
-        // slots whose rank falls in this round's window are staged
-        const int c0 = s_cs[0], c1 = s_cs[kP2GChunk];
-        auto cell_of_slot = [&](int slot) {
-          int lo = 0;  // the cell of this slot: the last cell whose start is <= slot
-          if (slot - c0 < kP2GMap) {
-            lo = s_map[slot - c0];
-          } else {
-            int hi = kP2GChunk;
-            while (hi - lo > 1) {
-              const int mid = (lo + hi) >> 1;
-              if (s_cs[mid] <= slot) lo = mid;
-              else hi = mid;
-            }
-          }
-          return lo;
-        };
-        auto stage_one = [&](int cl, int r, const p2g_particle &pp) {
-          const int cell = cell0 + cl;
-          const int ex = (cell >> 6) + 1, ey = ((cell >> 3) & 7) + 1, ez = (cell & 7) + 1;
-          if (pp.hb[0] != ex || pp.hb[1] != ey || pp.hb[2] != ez) {
-            // a stencil origin that rounding moved off the cell: this particle by itself, and a
-            // zero-mass stand-in in its staging place
-            p2g_direct(s, sh, pp, b);
-            for (int f = 0; f < kP2GVec; ++f) stg[f][r][cl] = make_float4(0.f, 0.f, 0.f, 0.f);
-            return;
-          }
-          if (kP2GStageF) {
-            stg[0][r][cl] = make_float4(pp.f[0], pp.f[1], pp.f[2], pp.m);
-          } else {
-            stg[0][r][cl] = make_float4(pp.w[0][0], pp.w[0][1], pp.w[0][2], pp.w[1][0]);
-            stg[1][r][cl] = make_float4(pp.w[1][1], pp.w[1][2], pp.w[2][0], pp.w[2][1]);
-            stg[2][r][cl] = make_float4(pp.w[2][2], pp.m, 0.f, 0.f);
-          }
+    auto copy = [&]() {
+      float4 *const d = cp_dst + fill * kP2GStage;
+      if (src0 >= 0) {
+        const float4 *const r = rows + row_at(0, src0);
+        cp_async16(d, s.cur.xm + src0);
+        cp_async16(d + kP2GField, r);
+        cp_async16(d + 2 * kP2GField, r + 32);
+        cp_async16(d + 3 * kP2GField, r + 64);
+      }
+      if (src1 >= 0) {
+        const float4 *const r = rows + row_at(0, src1);
+        cp_async16(d + 8, s.cur.xm + src1);
+        cp_async16(d + 8 + kP2GField, r);
+        cp_async16(d + 8 + 2 * kP2GField, r + 32);
+        cp_async16(d + 8 + 3 * kP2GField, r + 64);
+      }
+      cp_async_commit();
+      fill = fill + 1 == S ? 0 : fill + 1;
+    };
+    load_src();
 #pragma unroll
-          for (int d = 0; d < 3; ++d)
-            stg[kP2GQ + d][r][cl] = make_float4(pp.q[d], pp.ax[d], pp.ay[d], pp.az[d]);
-        };
-        for (int slot = c0 + t; slot < c1; slot += 2 * blockDim.x) {
-          const int slot2 = slot + blockDim.x;
-          const int cl1 = cell_of_slot(slot), r1 = slot - s_cs[cl1] - rlo;
-          const bool in1 = r1 >= 0 && r1 < R;
-          int cl2 = 0, r2 = -1;
-          if (slot2 < c1) {
-            cl2 = cell_of_slot(slot2);
-            r2 = slot2 - s_cs[cl2] - rlo;
-          }
-          const bool in2 = r2 >= 0 && r2 < R;
-          if (!in1 && !in2) continue;
-          p2g_raw ra, rb;
-          if (kPrefetchSrc) {
-            int src1, src2;
-            if (round == 0 && slot == c0 + t && pre1 >= 0) {
-              src1 = pre1;
-              src2 = slot2 < c1 ? pre2 : pre1;
-            } else {
-              src1 = s.src[slot];
-              src2 = slot2 < c1 ? s.src[slot2] : src1;
-            }
-            p2g_load(s, affine, in1 ? src1 : src2, ra);
-            p2g_load(s, affine, in2 ? src2 : src1, rb);
-          } else {
-            p2g_load(s, affine, s.src[in1 ? slot : slot2], ra);
-            p2g_load(s, affine, s.src[in2 ? slot2 : slot], rb);
-          }
-          p2g_particle pp;
-          if (in1) {
-            p2g_prepare<kCell>(s.prm, ra, ox, oy, oz, pp, with_mass != 0);
-            stage_one(cl1, r1, pp);
-          }
-          if (in2) {
-            p2g_prepare<kCell>(s.prm, rb, ox, oy, oz, pp, with_mass != 0);
-            stage_one(cl2, r2, pp);
-          }
-        }
-        __syncthreads();
-        if (last && chunk + 1 < 512 / kP2GChunk) fill(chunk + 1);
-        if (kPrefetchSrc) {
-          pre1 = pre2 = -1;
-          if (last && chunk + 1 < 512 / kP2GChunk) {
-            const int c0n = s.cell_start[b * 512 + (chunk + 1) * kP2GChunk];
-            const int c1n = chunk + 2 < 512 / kP2GChunk ? s.cell_start[b * 512 + (chunk + 2) * kP2GChunk] : end;
-            if (c0n + t < c1n) pre1 = s.src[c0n + t];
-            if (c0n + t + (int)blockDim.x < c1n) pre2 = s.src[c0n + t + blockDim.x];
-          }
-        }
-        // ---- phase 2: thread (cell, channel) sums the staged particles of its cell
-        const int cnt = min(s_cs[my_cell + 1] - s_cs[my_cell] - rlo, R);
-        if (cnt > 0) {
-          float acc[27];
+    for (int k = 0; k < S - 1; ++k) {
+      copy();
+      load_src();
+    }
+
+    float2 acc[27];
 #pragma unroll
-          for (int n = 0; n < 27; ++n) acc[n] = 0.f;
-          const int d = my_ch - 1;  // p channel index, -1 for mass
-          if (my_ch == 0) {
-            // mass: W m (the warp is channel-uniform)
-            for (int r = 0; r < cnt; ++r) {
-              float w[3][3], m;
-              staged_weights<kCell, R>(stg, r, my_cell, w, m);
-#pragma unroll
-              for (int ii = 0; ii < 3; ++ii) {
-                const float wm = w[0][ii] * m;
-#pragma unroll
-                for (int jj = 0; jj < 3; ++jj) {
-                  const float wij = wm * w[1][jj];
-#pragma unroll
-                  for (int kk = 0; kk < 3; ++kk) {
-                    const int n = (ii * 3 + jj) * 3 + kk;
-                    acc[n] = fmaf(wij, w[2][kk], acc[n]);
-                  }
-                }
+    for (int n = 0; n < 27; ++n) acc[n] = make_float2(0.f, 0.f);
+    int hot = 0;    // planes until the carried sums are all zero
+    int drain = 0;  // ring stage consumed next
+    // planes go two at a time: one barrier, and a warp may run ahead of the others within them
+#pragma unroll 1
+    for (int p0 = 0; p0 < nx + 2; p0 += 2) {
+      const float *const pl0 = plane + (p0 & 2) * 4 * kP2GPlane;
+      if (p0 == 2 && next_b >= 0) fetch_meta(meta + (par ^ 1) * kMeta, next_b);
+#pragma unroll 1
+      for (int p = p0; p < min(p0 + 2, nx + 2); ++p) {
+        if (p < nx) {
+          const int c = (x0 + p) * 64 + cell16;
+          const int cnt = mycells[c + 1] - mycells[c];
+          const int maxc = __reduce_max_sync(kFull, cnt);
+          const float bx = (float)(bk.x * 8 + x0 + p + 2);
+          if (maxc > 0) hot = 3;
+#pragma unroll 1
+          for (int r0 = 0; r0 < maxc; r0 += kP2GWin) {
+            cp_async_wait<S - 2>();
+            __syncwarp();  // the window has landed for every lane, the stage before it is free
+            copy();
+            load_src();
+            const float4 *const st = ring + drain * kP2GStage + cell16;
+            const float4 *const pa = pair ? st + 2 * kP2GField : unit;
+            const float4 *const pb = pair ? st + 3 * kP2GField : st + kP2GField;
+            drain = drain + 1 == S ? 0 : drain + 1;
+            const int rn = min(cnt - r0, kP2GWin);
+            float4 xm = st[0], ra = pa[0], rb = pb[0];
+#pragma unroll 1
+            for (int r = 0; r < rn; ++r) {
+              // the next rank's data load while this one is summed (the row behind the last is
+              // the next field's, read and not used)
+              const float4 xm_n = st[(r + 1) * kP2GRow], ra_n = pa[(r + 1) * kP2GRow], rb_n = pb[(r + 1) * kP2GRow];
+              float X[3];
+              if (kCell) {  // the index bucket floor(x * (1/dx) + 1/2) as the binning keys it
+                X[0] = xm.x * prm.inv_dx, X[1] = xm.y * prm.inv_dx, X[2] = xm.z * prm.inv_dx;
+              } else {
+                X[0] = over_dx(prm, xm.x), X[1] = over_dx(prm, xm.y), X[2] = over_dx(prm, xm.z);
               }
-            }
-          } else {
-            // momentum: W (q + ii ax + jj ay + kk az), in cell units of the node offset
-            for (int r = 0; r < cnt; ++r) {
-              float w[3][3], m_unused;
-              staged_weights<kCell, R>(stg, r, my_cell, w, m_unused);
-              const float4 qa = stg[kP2GQ + d][r][my_cell];
-              const float q = qa.x, ax = qa.y, ay = qa.z, az = qa.w;
-              // wz (qij + kk az) = wz qij + cz[kk], cz = (0, wz1 az, 2 wz2 az): two operations
-              // per node
-              const float cz1 = w[2][1] * az, cz2 = 2.f * w[2][2] * az;
+              const float2 hx = dup2(bx - X[0]), hy = dup2(by - X[1]), hz = dup2(bz - X[2]);
+              // W (qm + (ii - 1) ax + (jj - 1) ay + (kk - 1) az): qm the momentum the middle node
+              // would take, a the affine terms of one cell
+              const float2 ax = mul2(make_float2(ra.y, rb.y), dx8), ay = mul2(make_float2(ra.z, rb.z), dx8),
+                           az = mul2(make_float2(ra.w, rb.w), dx8);
+              float2 q = mul2(dup2(xm.w * mscale), make_float2(ra.x, rb.x));
+              q = fma2(ax, hx, q);
+              q = fma2(ay, hy, q);
+              q = fma2(az, hz, q);
+              float2 wx[3], wy[3], wz[3];
+              if (kCell) {
+                cell_weights2(hx, wx);
+                cell_weights2(hy, wy);
+                cell_weights2(hz, wz);
+              } else {
+                bspline_weights2(hx, wx);
+                bspline_weights2(hy, wy);
+                bspline_weights2(hz, wz);
+              }
+              const float2 minus = dup2(-1.f);
+              const float2 c0 = mul2(mul2(wz[0], az), minus), c2 = mul2(wz[2], az);
 #pragma unroll
               for (int ii = 0; ii < 3; ++ii) {
-                const float qi = q + (float)ii * ax;
+                const float2 qi = ii == 0 ? fma2(ax, minus, q) : ii == 1 ? q : add2(q, ax);
 #pragma unroll
                 for (int jj = 0; jj < 3; ++jj) {
-                  const float qij = qi + (float)jj * ay;
-                  const float wij = w[0][ii] * w[1][jj];
+                  const float2 qij = jj == 0 ? fma2(ay, minus, qi) : jj == 1 ? qi : add2(qi, ay);
+                  const float2 wij = mul2(wx[ii], wy[jj]);
                   const int n = (ii * 3 + jj) * 3;
-                  acc[n] = fmaf(wij, w[2][0] * qij, acc[n]);
-                  acc[n + 1] = fmaf(wij, fmaf(w[2][1], qij, cz1), acc[n + 1]);
-                  acc[n + 2] = fmaf(wij, fmaf(w[2][2], qij, cz2), acc[n + 2]);
+                  acc[n] = fma2(wij, fma2(wz[0], qij, c0), acc[n]);
+                  acc[n + 1] = fma2(wij, mul2(wz[1], qij), acc[n + 1]);
+                  acc[n + 2] = fma2(wij, fma2(wz[2], qij, c2), acc[n + 2]);
                 }
               }
+              xm = xm_n, ra = ra_n, rb = rb_n;
             }
           }
-          // cell (lx, ly, lz): stencil origin (lx + 1, ly + 1, lz + 1) from 8b, halo node
-          // (lx, ly, lz + 1)
-          const int cell = cell0 + my_cell;
-          const int hx = cell >> 6, hy = (cell >> 3) & 7, hz = (cell & 7) + 1;
-          float *dst = sh + my_ch * kP2GHaloNodes;
-#pragma unroll
-          for (int ii = 0; ii < 3; ++ii)
-#pragma unroll
-            for (int jj = 0; jj < 3; ++jj)
-#pragma unroll
-              for (int kk = 0; kk < 3; ++kk)
-                atomicAdd(&dst[((hx + ii) * kP2GHy + (hy + jj)) * kP2GHz + hz + kk], acc[(ii * 3 + jj) * 3 + kk]);
         }
-        if (last) break;
+        // ---- the plane's leading nodes (x0 + p + 1 from 8b) are complete for this column: the
+        // warp adds its lanes' 3 x 3 sums up into its 4 rows of 10 nodes by shuffles and stores
+        // them (every entry has one writer, so no atomics and nothing to clear)
+        if (lane == 0) s_hot[(p0 & 2) + (p & 1)][w] = hot > 0;
+        if (hot > 0) {
+          --hot;
+          float2 lo[3], hi[3];  // of row y + jj: node z + kk summed over the lanes at z; nodes 8 and 9 past lanes 6, 7
+#pragma unroll
+          for (int jj = 0; jj < 3; ++jj) {
+            const float2 a0 = acc[3 * jj], a1 = acc[3 * jj + 1], a2 = acc[3 * jj + 2];
+            const float2 u1 = shfl_up2(a1, 1), u2 = shfl_up2(a2, 2), d1 = shfl_down2(a1, 1);
+            lo[jj] = a0;
+            if (lz >= 1) lo[jj] = add2(lo[jj], u1);
+            if (lz >= 2) lo[jj] = add2(lo[jj], u2);
+            hi[jj] = lz == 6 ? add2(a2, d1) : a2;  // used by lanes 6 and 7
+          }
+          // the two y rows of the warp: lanes of the first end with rows 0 and 1, of the second 2 and 3
+          const bool second = (ly & 1) != 0;
+          const float2 xl = shfl_xor2(second ? lo[0] : lo[2], 8), xh = shfl_xor2(second ? hi[0] : hi[2], 8);
+          const float2 r0 = second ? add2(lo[1], xl) : lo[0], r1 = second ? lo[2] : add2(lo[1], xl);
+          const float2 h0 = second ? add2(hi[1], xh) : hi[0], h1 = second ? hi[2] : add2(hi[1], xh);
+          float *const e = emit0 + ((p0 & 2) + (p & 1)) * 4 * kP2GPlane;
+          e[0] = r0.x;
+          e[kP2GPlaneCh] = r0.y;
+          e[kP2GPlaneRow] = r1.x;
+          e[kP2GPlaneCh + kP2GPlaneRow] = r1.y;
+          if (lz >= 6) {
+            e[2] = h0.x;
+            e[kP2GPlaneCh + 2] = h0.y;
+            e[kP2GPlaneRow + 2] = h1.x;
+            e[kP2GPlaneCh + kP2GPlaneRow + 2] = h1.y;
+          }
+#pragma unroll
+          for (int n = 0; n < 18; ++n) acc[n] = acc[n + 9];
+#pragma unroll
+          for (int n = 18; n < 27; ++n) acc[n] = make_float2(0.f, 0.f);
+        }
+      }
+      __syncthreads();
+      // ---- flush the two planes: each 4 channels x 10 y x 3 quads of z, a row summed over the two
+      // warps that share it, by 16-byte reductions into the blocks b + {0,1}^3; the next two planes
+      // go to the other buffers, so one barrier is enough
+      for (int it = t; it < 120 * min(2, nx + 2 - p0); it += kP2GThreads) {
+        const int p = it < 120 ? 0 : 1, u = it - 120 * p;
+        const int ch = u / 30, hy = u % 30 / 3, quad = u % 3;
+        const float *const at = pl0 + p * 4 * kP2GPlane + ch * kP2GPlaneCh + quad * 4;
+        const int v = hy >> 1, row = hy & 1;
+        float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (v < 4 && s_hot[(p0 & 2) + p][v])
+          q4 = *reinterpret_cast<const float4 *>(at + v * kP2GPlane + row * kP2GPlaneRow);
+        if (v > 0 && s_hot[(p0 & 2) + p][v - 1]) {
+          const float4 o = *reinterpret_cast<const float4 *>(at + (v - 1) * kP2GPlane + (row + 2) * kP2GPlaneRow);
+          q4.x += o.x, q4.y += o.y, q4.z += o.z, q4.w += o.w;
+        }
+        if (q4.x != 0.f || q4.y != 0.f || q4.z != 0.f || q4.w != 0.f) {
+          const int X = x0 + p0 + p + 1, Y = hy + 1;
+          const int tb = cs[kMetaNbr + ((X >= 8 ? 4 : 0) | (Y >= 8 ? 2 : 0) | (quad == 2 ? 1 : 0))];
+          if (tb < 0)
+            set_status(s.ctr, kStatusMissingBlock);
+          else
+            red_add_v4(s.grid + ((size_t)tb * kGridChannels + ch) * 512 +
+                           (((X & 7) << 6) | ((Y & 7) << 3) | ((quad * 4) & 7)),
+                       q4.x, q4.y, q4.z, q4.w);
+        }
       }
     }
-    __syncthreads();
-    // flush: items (ch, hx, hy, quad) over 4 x 10 x 10 x 3; halo node (hx, hy, 4 quad + j) is
-    // the grid cell (8b + 1 + hx, 8b + 1 + hy, 8b + 4 quad + j)
-    for (int it = t; it < kGridChannels * kP2GHx * kP2GHy * 3; it += blockDim.x) {
-      const int quad = it % 3, hy = (it / 3) % kP2GHy, hx = (it / (3 * kP2GHy)) % kP2GHx,
-                ch = it / (3 * kP2GHy * kP2GHx);
-      float4 *src4 = reinterpret_cast<float4 *>(&sh[((ch * kP2GHx + hx) * kP2GHy + hy) * kP2GHz + quad * 4]);
-      const float4 q4 = *src4;
-      if (q4.x == 0.f && q4.y == 0.f && q4.z == 0.f && q4.w == 0.f) continue;
-      *src4 = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int X = hx + 1, Y = hy + 1;
-      const int tt = (X >= 8 ? 4 : 0) | (Y >= 8 ? 2 : 0) | (quad == 2 ? 1 : 0);
-      const int tb = s.nbr[b * 8 + tt];
-      if (tb < 0) {
-        set_status(s.ctr, kStatusMissingBlock);
-        continue;
-      }
-      const int cell = ((X & 7) << 6) | ((Y & 7) << 3) | ((quad * 4) & 7);
-      red_add_v4(s.grid + ((size_t)tb * kGridChannels + ch) * 512 + cell, q4.x, q4.y, q4.z, q4.w);
-    }
+    item = next;
   }
 }
 
@@ -1263,7 +1270,7 @@ __device__ __forceinline__ float cell_dinv(const scene_params &p, float x) {
 // The pair's per-particle affine term A of the stored state, in the particle order of cur:
 // part 0 the whole term (P2C2GTransfer; the cell-scheme counterpart of k_prime), 1 the momentum
 // part m B Dinv (P2C2GTransferMomentum), 2 the force part -dt V0 P F^T Dinv (P2C2GTransferForce).
-__global__ void __launch_bounds__(kThreads) k_cell_affine(scene_device s, int part, float *out) {
+__global__ void __launch_bounds__(kThreads) k_cell_affine(scene_device s, int part, float4 *out) {
   if (part == 0 && blockIdx.x == 0 && threadIdx.x == 0) s.ctr[kCtrMaskFrom] = 0;
   const scene_params &p = s.prm;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += grid_threads()) {
@@ -1273,13 +1280,17 @@ __global__ void __launch_bounds__(kThreads) k_cell_affine(scene_device s, int pa
 #pragma unroll
     for (int k = 0; k < 9; ++k) F[k] = s.cur.F[mat_at(k, i)];
     float pl = 0.f;
-    if (part != 1) constitutive(p.mat, F, pl, tau);
+    if (part != 1) constitutive_update<false, true>(p.mat, F, pl, tau);
+    float A[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const float mB = part == 2 ? 0.f : xm.w * s.cur.C[mat_at(k, i)];
       const float f = part == 1 ? 0.f : p.dt * tau[k];
-      out[mat_at(k, i)] = (mB - f) * dinv[k / 3];
+      A[k] = (mB - f) * dinv[k / 3];
     }
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      out[row_at(d, i)] = make_float4(s.cur.row[row_at(d, i)].x, A[d], A[3 + d], A[6 + d]);
   }
 }
 
@@ -1400,6 +1411,26 @@ __device__ __forceinline__ principal_result plain_principal(const material_dev &
   return snow_principal(mat.mu, mat.lambda, mat.hardening, mat.theta_c, mat.theta_s, S, plastic);
 }
 
+// columns i and j of (log S, S, U, V) by descending singular value
+__device__ __forceinline__ void sort_columns(float *l, float *S, float *U, float *V, int i, int j) {
+  if (S[i] >= S[j]) return;
+  float t = S[i];
+  S[i] = S[j];
+  S[j] = t;
+  t = l[i];
+  l[i] = l[j];
+  l[j] = t;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    t = U[3 * i + r];
+    U[3 * i + r] = U[3 * j + r];
+    U[3 * j + r] = t;
+    t = V[3 * i + r];
+    V[3 * i + r] = V[3 * j + r];
+    V[3 * j + r] = t;
+  }
+}
+
 // The learned constitutive update (committed ordering), G2P's part.
 //
 // The network replaces the return-mapping branch, i.e. the projection of a trial state that
@@ -1419,7 +1450,10 @@ __device__ __forceinline__ bool learned_update(const scene_device &s, const mate
                                                float *F, float &plastic, float *tau, bool active, int slot, int sid,
                                                int id, float m, const float *Cm, unsigned &all_updates) {
   float U[9], S[3], V[9];
-  svd3<true>(F, U, S, V);
+  bool columns = false;
+  if (mat.model == 1) columns = svd3_columns<true>(F, U, S, V);
+  const unsigned rest = __ballot_sync(kFull, !columns);
+  if (!columns) svd3<true>(F, U, S, V, rest);
   float feat[6];
   closure_features(mat, S, plastic, feat);
   bool project = false;
@@ -1452,13 +1486,19 @@ __device__ __forceinline__ bool learned_update(const scene_device &s, const mate
       H[i] = feat[i];
     }
   }
+  // the network takes the log singular values in descending order, as svd3 sorts them
+  if (project && columns) {
+    sort_columns(feat, S, U, V, 0, 1);
+    sort_columns(feat, S, U, V, 0, 2);
+    sort_columns(feat, S, U, V, 1, 2);
+  }
   bool in_hull = true;
 #pragma unroll
   for (int k = 0; k < kMlpIn; ++k) in_hull = in_hull && feat[k] >= cd.in_min[k] && feat[k] <= cd.in_max[k];
   bool queued = false;
   const bool want = active && project && in_hull;
-  const unsigned wq = __ballot_sync(0xffffffffu, want);
-  all_updates += __popc(__ballot_sync(0xffffffffu, active));
+  const unsigned wq = __ballot_sync(kFull, want);
+  all_updates += __popc(__ballot_sync(kFull, active));
   if (wq) {
     const int lane = threadIdx.x & 31;
     int base = 0;
@@ -1603,9 +1643,12 @@ __global__ void __launch_bounds__(kThreads) k_closure_finish(scene_device s) {
     mul_diag_t(Fn, U, Ns, V);
     const float m = u[22];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) {
-      s.nxt.F[mat_at(c, slot)] = Fn[c];
-      s.nxt.A[mat_at(c, slot)] = m * u[23 + c] - s.prm.kappa * tau[c];
+    for (int c = 0; c < 9; ++c) s.nxt.F[mat_at(c, slot)] = Fn[c];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {  // (the row's first entry is the velocity, which G2P wrote)
+      float *const r = &s.nxt.row[row_at(d, slot)].x;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) r[1 + c] = m * u[23 + 3 * c + d] - s.prm.kappa * tau[3 * c + d];
     }
     if (s.nxt.plastic) s.nxt.plastic[slot] = pl_new;
   }
@@ -1619,18 +1662,6 @@ constexpr int kG2PPrefetch = 4 * 32 + 9 * 32 + 32 + 32;
 constexpr size_t g2p_smem_bytes(int nt) {
   return sizeof(float4) * kHaloCells + sizeof(float) * 2 * kG2PPrefetch * (size_t)(nt / 32);
 }
-
-// cp.async (sm_80 and later): copies that land in shared memory while the warp computes
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(a), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
 // kLearned: the closure's network gives the return map's projections (queued for the tcgen05
 // pass, 256 threads only); kBatch: batched scenes (per-block scene material, scene-local block
@@ -1654,7 +1685,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 5) k_g2p(scene_device s) {
   __shared__ material_dev s_mat;
   __shared__ unsigned s_moved;  // the block's move mask
   const scene_params &p = s.prm;
-  const int nb = s.ctr[kCtrBlocks];
+  const int nb = s.ctr[kCtrBlocks], front = s.ctr[kCtrOrderFront], nwork = work_blocks(s);
+  const int parts = slot_parts(nwork, gridDim.x);
   const int substep = s.ctr[kCtrSubstep];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     s.ctr[kCtrMaskFrom] = nb;
@@ -1676,13 +1708,13 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 5) k_g2p(scene_device s) {
   };
   for (;;) {
     const int w = grab_block(&s.ctr[kCtrWork + kWorkG2P], &s_b);
-    if (w >= nb) break;
-    const int b = s.work_order[w];
-    const int start = s.block_start[b], end = s.block_start[b + 1];
-    if (start == end) {
-      if (threadIdx.x == 0) s.bmask[b] = 0u;
-      continue;
-    }
+    if (w >= nwork * parts) break;
+    const int b = work_block(s, front, nb, w / parts);
+    // this item's part of the block's slots
+    const int first = s.block_start[b], last = s.block_start[b + 1];
+    const int len = (last - first + 32 * parts - 1) / (32 * parts) * 32;
+    const int start = first + w % parts * len, end = min(last, start + len);
+    if (start >= end) continue;
     const int3 gk = unpack_key(s.blk_pk[b]);
     if (kBatch && threadIdx.x == 0) s_mat = p.mats[scene_of_key(gk)];
     if (threadIdx.x == 0) s_moved = 0u;
@@ -1770,8 +1802,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 5) k_g2p(scene_device s) {
       if (active && !inside) set_status(s.ctr, kStatusMissingBlock);
       // the cell this slot was binned in, as the binning computed it from the same position
       const int sid = kBatch ? s.cur.sid[icur] : 0;
-      int3 cell_old = make_int3(0x7fffffff, 0, 0), blk_old;
-      if (active && !particle_cell(s, sid, xm, cell_old, blk_old)) cell_old.x = 0x7fffffff;
+      const float cold[3] = {floorf(bucket_of(p, xm.x)), floorf(bucket_of(p, xm.y)), floorf(bucket_of(p, xm.z))};
       float vel[3] = {0.f, 0.f, 0.f};
       float B[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // sum W v (node - f)^T
       if (inside) {
@@ -1844,22 +1875,25 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 5) k_g2p(scene_device s) {
         // the block of the new position, as the next activation computes it from the stored
         // x, recorded relative to this block for k_insert_moved_blocks; and whether the
         // particle left the cell it was binned in, for the next (incremental) binning
-        unsigned bit = 0u;
-        bool moved_far = false, left_cell = false;
-        if (active) {
+        // (most particles stay in their cell, where the block is this one)
+        unsigned bit = active ? 1u << 13 : 0u;
+        bool moved_far = false;
+        const bool left_cell = active && !(floorf(bucket_of(p, xm.x)) == cold[0] &&
+                                           floorf(bucket_of(p, xm.y)) == cold[1] &&
+                                           floorf(bucket_of(p, xm.z)) == cold[2]);
+        if (left_cell) {
           int3 c2, b2;
+          bit = 0u;
+          moved_far = true;
           if (particle_cell(s, sid, xm, c2, b2)) {
             const int ox = b2.x - gk.x, oy = b2.y - gk.y, oz = b2.z - gk.z;
-            if (ox >= -1 && ox <= 1 && oy >= -1 && oy <= 1 && oz >= -1 && oz <= 1)
+            if (ox >= -1 && ox <= 1 && oy >= -1 && oy <= 1 && oz >= -1 && oz <= 1) {
               bit = 1u << ((ox + 1) * 9 + (oy + 1) * 3 + (oz + 1));
-            else
-              moved_far = true;
-            left_cell = c2.x != cell_old.x || c2.y != cell_old.y || c2.z != cell_old.z;
-          } else {
-            moved_far = true;  // the particle pass of the next activation reports it
-          }
-          s.moved[slot] = (uint8_t)(left_cell || moved_far);
+              moved_far = false;
+            }
+          }  // (else the particle pass of the next activation reports it)
         }
+        if (active) s.moved[slot] = (uint8_t)left_cell;
         const unsigned wbits = __reduce_or_sync(kFull, bit);
         if (lane == 0 && wbits) atomicOr(&s_moved, wbits);
         bool bad = moved_far;
@@ -1911,37 +1945,42 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 5) k_g2p(scene_device s) {
       if (kLearned && (!kBatch || s_mat.model == s.aux.cd.model))
         queued = learned_update(s, kBatch ? s_mat : p.mat, s.aux.cd, Fn, pl, tau, active, slot, sid, id, xm.w, C,
                                 all_updates);
-      else if (kBatch)
-        constitutive<true>(s_mat, Fn, pl, tau);
       else
-        constitutive<true>(p.mat, Fn, pl, tau);
+        constitutive_update<true, true>(kBatch ? s_mat : p.mat, Fn, pl, tau);
       if (!active) continue;
       s.nxt.xm[slot] = xm;
-      s.nxt.v[slot] = make_float4(vel[0], vel[1], vel[2], 0.f);
+      if (p.store_c) {
 #pragma unroll
-      for (int k = 0; k < 9; ++k) s.nxt.C[mat_at(k, slot)] = C[k];
+        for (int k = 0; k < 9; ++k) s.nxt.C[mat_at(k, slot)] = C[k];
+      }
       if (kCell) {
         // the affine term of the next P2C2G, from the new position and F (P2C2G.hpp:86-146)
         const float dnew[3] = {cell_dinv(p, xm.x), cell_dinv(p, xm.y), cell_dinv(p, xm.z)};
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-          s.nxt.A[mat_at(k, slot)] = (xm.w * C[k] - p.dt * tau[k]) * dnew[k / 3];
-          s.nxt.F[mat_at(k, slot)] = Fn[k];
-        }
-        if (s.nxt.plastic) s.nxt.plastic[slot] = pl;
+        for (int d = 0; d < 3; ++d)
+          s.nxt.row[row_at(d, slot)] = make_float4(vel[d], (xm.w * C[d] - p.dt * tau[d]) * dnew[0],
+                                                   (xm.w * C[3 + d] - p.dt * tau[3 + d]) * dnew[1],
+                                                   (xm.w * C[6 + d] - p.dt * tau[6 + d]) * dnew[2]);
       } else if (!queued) {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-          s.nxt.A[mat_at(k, slot)] = xm.w * C[k] - p.kappa * tau[k];
-          s.nxt.F[mat_at(k, slot)] = Fn[k];
-        }
+        for (int d = 0; d < 3; ++d)
+          s.nxt.row[row_at(d, slot)] =
+              make_float4(vel[d], xm.w * C[d] - p.kappa * tau[d], xm.w * C[3 + d] - p.kappa * tau[3 + d],
+                          xm.w * C[6 + d] - p.kappa * tau[6 + d]);
+      } else {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s.nxt.row[row_at(d, slot)].x = vel[d];
+      }
+      if (!queued) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) s.nxt.F[mat_at(k, slot)] = Fn[k];
         if (s.nxt.plastic) s.nxt.plastic[slot] = pl;
       }
       s.nxt.id[slot] = id;
       if (kBatch) s.nxt.sid[slot] = sid;
     }
     __syncthreads();
-    if (threadIdx.x == 0) s.bmask[b] = s_moved;
+    if (threadIdx.x == 0 && s_moved) atomicOr(&s.bmask[b], s_moved);
   }
   if (kLearned && lane == 0 && all_updates) atomicAdd(&s.aux.cd.audit[7], (double)all_updates);
 }
@@ -1985,7 +2024,7 @@ __global__ void __launch_bounds__(kG2P2GThreads, 2)
   unsigned char *const s_map0 = reinterpret_cast<unsigned char *>(s_cs0 + 2 * (kG2P2GChunk + 1));
   __shared__ int s_b;
   const scene_params &p = s.prm;
-  const int nb = s.ctr[kCtrBlocks];
+  const int nb = s.ctr[kCtrBlocks], front = s.ctr[kCtrOrderFront], nwork = work_blocks(s);
   if ((long long)nb * 1536 > ndofs) {
     if (blockIdx.x == 0 && threadIdx.x == 0) set_status(s.ctr, kStatusCapacity);
     return;
@@ -1996,10 +2035,9 @@ __global__ void __launch_bounds__(kG2P2GThreads, 2)
   for (int q = t; q < 3 * kHaloCells; q += kG2P2GThreads) sf[q] = 0.f;
   for (;;) {
     const int w = grab_block(&s.ctr[kCtrWork + kWorkG2P2G], &s_b);
-    if (w >= nb) break;
-    const int b = s.work_order[w];
-    const int start = s.block_start[b], end = s.block_start[b + 1];
-    if (start == end) continue;
+    if (w >= nwork) break;
+    const int b = work_block(s, front, nb, w);
+    const int end = s.block_start[b + 1];
     // velocity halo: items (hx, hy, quad) over 12 x 12 x 3; four consecutive nodes are 12
     // consecutive floats (three 16-byte loads)
     for (int it = t; it < kHalo * kHalo * 3; it += kG2P2GThreads) {
@@ -2113,7 +2151,7 @@ __global__ void __launch_bounds__(kG2P2GThreads, 2)
             Fn[3 * c + r] = F[3 * c + r] + dt * p.four_over_dx *
                                                (B[r] * F[3 * c] + B[3 + r] * F[3 * c + 1] + B[6 + r] * F[3 * c + 2]);
         float tau[9];
-        constitutive<true>(p.mat, Fn, pl, tau);
+        constitutive_update<true, false>(p.mat, Fn, pl, tau);
         if (!active) continue;
         float ax[3], ay[3], az[3], q[3];
 #pragma unroll
@@ -2432,8 +2470,10 @@ __global__ void k_import(scene_device s, const float *m, const float *x, const f
       model = s.prm.mats[sc].model;
     }
     const float plastic_default = model == 2 ? 1.f : 0.f;
-    s.cur.xm[i] = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], m[i]);
-    s.cur.v[i] = v ? make_float4(v[3 * i], v[3 * i + 1], v[3 * i + 2], 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+    s.cur.xm[i] = make_float4(x[3 * (size_t)i], x[3 * (size_t)i + 1], x[3 * (size_t)i + 2], m[i]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      s.cur.row[row_at(d, i)] = make_float4(v ? v[3 * (size_t)i + d] : 0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       s.cur.C[mat_at(k, i)] = C ? C[9 * (size_t)i + k] : 0.f;
@@ -2451,7 +2491,8 @@ __global__ void k_import_tv(scene_device s, const float *base, int nchn, int om,
     const size_t tile = (size_t)(i / 32) * nchn * 32 + (i % 32);
     auto at = [&](int chn) { return base[tile + (size_t)chn * 32]; };
     s.cur.xm[i] = make_float4(at(ox), at(ox + 1), at(ox + 2), at(om));
-    s.cur.v[i] = ov >= 0 ? make_float4(at(ov), at(ov + 1), at(ov + 2), 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s.cur.row[row_at(d, i)] = make_float4(ov >= 0 ? at(ov + d) : 0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       s.cur.C[mat_at(k, i)] = oC >= 0 ? at(oC + k) : 0.f;
@@ -2471,15 +2512,19 @@ __global__ void k_prime(scene_device s) {
     for (int k = 0; k < 9; ++k) F[k] = s.cur.F[mat_at(k, i)];
     float pl = s.cur.plastic ? s.cur.plastic[i] : 0.f;
     if (s.prm.batch)
-      constitutive(s.prm.mats[s.cur.sid[i]], F, pl, tau);
+      constitutive_update<false, true>(s.prm.mats[s.cur.sid[i]], F, pl, tau);
     else
-      constitutive(s.prm.mat, F, pl, tau);
+      constitutive_update<false, true>(s.prm.mat, F, pl, tau);
     const float m = s.cur.xm[i].w;
+    float A[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       s.cur.F[mat_at(k, i)] = F[k];
-      s.cur.A[mat_at(k, i)] = m * s.cur.C[mat_at(k, i)] - s.prm.kappa * tau[k];
+      A[k] = m * s.cur.C[mat_at(k, i)] - s.prm.kappa * tau[k];
     }
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      s.cur.row[row_at(d, i)] = make_float4(s.cur.row[row_at(d, i)].x, A[d], A[3 + d], A[6 + d]);
     if (s.cur.plastic) s.cur.plastic[i] = pl;
   }
 }
@@ -2487,7 +2532,8 @@ __global__ void k_prime(scene_device s) {
 __global__ void k_export(scene_device s, float *m, float *x, float *v, float *C, float *F, float *pl) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.prm.n; i += grid_threads()) {
     const int o = s.cur.id[i];
-    const float4 xm = s.cur.xm[i], vv = s.cur.v[i];
+    const float4 xm = s.cur.xm[i];
+    const float vv[3] = {s.cur.row[row_at(0, i)].x, s.cur.row[row_at(1, i)].x, s.cur.row[row_at(2, i)].x};
     if (m) m[o] = xm.w;
     if (x) {
       x[3 * (size_t)o] = xm.x;
@@ -2495,9 +2541,9 @@ __global__ void k_export(scene_device s, float *m, float *x, float *v, float *C,
       x[3 * (size_t)o + 2] = xm.z;
     }
     if (v) {
-      v[3 * (size_t)o] = vv.x;
-      v[3 * (size_t)o + 1] = vv.y;
-      v[3 * (size_t)o + 2] = vv.z;
+      v[3 * (size_t)o] = vv[0];
+      v[3 * (size_t)o + 1] = vv[1];
+      v[3 * (size_t)o + 2] = vv[2];
     }
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
@@ -2514,7 +2560,8 @@ __global__ void k_export_tv(scene_device s, float *base, int nchn, int om, int o
     const int o = s.cur.id[i];
     const size_t tile = (size_t)(o / 32) * nchn * 32 + (o % 32);
     auto at = [&](int chn) -> float & { return base[tile + (size_t)chn * 32]; };
-    const float4 xm = s.cur.xm[i], vv = s.cur.v[i];
+    const float4 xm = s.cur.xm[i];
+    const float vv[3] = {s.cur.row[row_at(0, i)].x, s.cur.row[row_at(1, i)].x, s.cur.row[row_at(2, i)].x};
     if (om >= 0) at(om) = xm.w;
     if (ox >= 0) {
       at(ox) = xm.x;
@@ -2522,9 +2569,9 @@ __global__ void k_export_tv(scene_device s, float *base, int nchn, int om, int o
       at(ox + 2) = xm.z;
     }
     if (ov >= 0) {
-      at(ov) = vv.x;
-      at(ov + 1) = vv.y;
-      at(ov + 2) = vv.z;
+      at(ov) = vv[0];
+      at(ov + 1) = vv[1];
+      at(ov + 2) = vv[2];
     }
     for (int k = 0; k < 9; ++k) {
       if (oC >= 0) at(oC + k) = s.cur.C[mat_at(k, i)];
@@ -2712,12 +2759,12 @@ cudaError_t prepare_kernels() {
       e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p2g_smem_bytes(ranks));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   };
-  p2g_attrs((const void *)k_p2g<false, 8, 4>, 8);
-  p2g_attrs((const void *)k_p2g<false, 12, 3>, 12);
-  p2g_attrs((const void *)k_p2g<false, 16, 2>, 16);
-  p2g_attrs((const void *)k_p2g<true, 8, 4>, 8);
-  p2g_attrs((const void *)k_p2g<true, 12, 3>, 12);
-  p2g_attrs((const void *)k_p2g<true, 16, 2>, 16);
+  p2g_attrs((const void *)k_p2g<false, 2>, 8);
+  p2g_attrs((const void *)k_p2g<false, 3>, 12);
+  p2g_attrs((const void *)k_p2g<false, 4>, 16);
+  p2g_attrs((const void *)k_p2g<true, 2>, 8);
+  p2g_attrs((const void *)k_p2g<true, 3>, 12);
+  p2g_attrs((const void *)k_p2g<true, 4>, 16);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_g2p2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG2P2GSmem);
   if (e != cudaSuccess) return e;
@@ -2746,35 +2793,35 @@ cudaError_t prepare_kernels() {
                               (int)g2p_smem_bytes(128));
 }
 
-// the staged P2G kernel of the scene's staging depth (p2g_ranks: 8, 12 or 16; 0 = 12)
+// the P2G kernel of the scene's staging depth (p2g_ranks: 8, 12 or 16)
 template <bool kCell>
-static void launch_staged_p2g(scene_device &s, const float *affine, int with_mass, cudaStream_t st) {
+static void launch_staged_p2g(scene_device &s, const float4 *rows, int with_mass, cudaStream_t st) {
   const int ranks = s.prm.p2g_ranks > 0 ? s.prm.p2g_ranks : kP2GRanksDefault;
   const int dflt = ranks == 8 ? 4 : ranks == 16 ? 2 : 3;
   const int grid = num_sms() * (s.prm.p2g_ctas_per_sm > 0 ? s.prm.p2g_ctas_per_sm : dflt);
   if (ranks == 8)
-    k_p2g<kCell, 8, 4><<<grid, kP2GThreads, p2g_smem_bytes(8), st>>>(s, affine, with_mass);
+    k_p2g<kCell, 2><<<grid, kP2GThreads, p2g_smem_bytes(8), st>>>(s, rows, with_mass);
   else if (ranks == 16)
-    k_p2g<kCell, 16, 2><<<grid, kP2GThreads, p2g_smem_bytes(16), st>>>(s, affine, with_mass);
+    k_p2g<kCell, 4><<<grid, kP2GThreads, p2g_smem_bytes(16), st>>>(s, rows, with_mass);
   else
-    k_p2g<kCell, 12, 3><<<grid, kP2GThreads, p2g_smem_bytes(12), st>>>(s, affine, with_mass);
+    k_p2g<kCell, 3><<<grid, kP2GThreads, p2g_smem_bytes(12), st>>>(s, rows, with_mass);
 }
 
 cudaError_t launch_p2g(scene_device &s, cudaStream_t st) {
   if (s.prm.transfer == kTransferCell) return launch_p2c2g(s, 0, st);
-  launch_staged_p2g<false>(s, s.cur.A, 1, st);
+  launch_staged_p2g<false>(s, s.cur.row, 1, st);
   return cudaGetLastError();
 }
 
 // part 0: P2C2GTransfer from the stored affine term; 1 (momentum) and 2 (force): the part's
-// affine term is formed first, into the next buffer's A (G2C2P rewrites it)
+// affine term is formed first, into the next buffer's rows (G2C2P rewrites them)
 cudaError_t launch_p2c2g(scene_device &s, int part, cudaStream_t st) {
-  const float *affine = s.cur.A;
+  const float4 *rows = s.cur.row;
   if (part != 0) {
-    k_cell_affine<<<num_sms() * 4, kThreads, 0, st>>>(s, part, s.nxt.A);
-    affine = s.nxt.A;
+    k_cell_affine<<<num_sms() * 4, kThreads, 0, st>>>(s, part, s.nxt.row);
+    rows = s.nxt.row;
   }
-  launch_staged_p2g<true>(s, affine, part == 2 ? 0 : 1, st);
+  launch_staged_p2g<true>(s, rows, part == 2 ? 0 : 1, st);
   return cudaGetLastError();
 }
 
@@ -2893,10 +2940,10 @@ cudaError_t launch_cg_iteration(scene_device &s, float *x, const cg_vectors &v, 
   return cudaGetLastError();
 }
 
-// k_begin, the two particle-block inserts (one returns at once), enlarge, prepare, set, 3 scans,
-// ranks, neighbours; the binning's 14 launches (the full and the incremental path, one of
-// which returns at once); p2g; grid update and boundaries; g2p
-int kernels_per_substep() { return 11 + 14 + 4; }
+// k_begin, the two particle-block inserts (one returns at once), enlarge, prepare, set,
+// 3 scans, ranks, neighbours; the binning's 14 launches (the full and the incremental path, one of
+// which returns at once).  Then p2g; grid update and boundaries; g2p
+int kernels_per_substep(const scene_device &) { return 11 + 14 + 4; }
 
 cudaError_t launch_import(scene_device &s, const float *m, const float *x, const float *v,
                           const float *C, const float *F, const float *plastic, int n,
@@ -2915,7 +2962,7 @@ cudaError_t launch_import_tilevector(scene_device &s, const float *base, int nch
 
 cudaError_t launch_prime(scene_device &s, cudaStream_t st) {
   if (s.prm.transfer == kTransferCell)
-    k_cell_affine<<<num_sms() * 4, kThreads, 0, st>>>(s, 0, s.cur.A);
+    k_cell_affine<<<num_sms() * 4, kThreads, 0, st>>>(s, 0, s.cur.row);
   else
     k_prime<<<num_sms() * 4, kThreads, 0, st>>>(s);
   return cudaGetLastError();
