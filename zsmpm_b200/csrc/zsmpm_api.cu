@@ -318,10 +318,14 @@ zsmpm_status substep_enqueue(zsmpm_scene *s, cudaStream_t st, bool defer_closure
   bind_buffers(s);
   if (s->timing) cudaEventRecord(s->ev[0], st);
   s->dev.prm.bin_full = 0;
-  ZS_TRY(launch_activate(s->dev, st), "activate");
-  if (s->timing) cudaEventRecord(s->ev[1], st);
-  ZS_TRY(launch_bin(s->dev, st), "bin");
-  if (s->timing) cudaEventRecord(s->ev[2], st);
+  if (fused_prepare(s->dev) && !s->timing) {
+    ZS_TRY(launch_prepare(s->dev, true, true, st), "activate and bin");
+  } else {
+    ZS_TRY(launch_activate(s->dev, st), "activate");
+    if (s->timing) cudaEventRecord(s->ev[1], st);
+    ZS_TRY(launch_bin(s->dev, st), "bin");
+    if (s->timing) cudaEventRecord(s->ev[2], st);
+  }
   if (s->join_pending) {
     // the last substep's closure pass writes F, the affine momentum and the plastic state that
     // this P2G and G2P read

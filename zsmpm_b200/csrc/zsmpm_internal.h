@@ -197,6 +197,9 @@ cudaError_t launch_grid_update(scene_device &s, cudaStream_t st);
 cudaError_t launch_g2p(scene_device &s, cudaStream_t st, bool closure_pass = true);
 cudaError_t launch_closure_pass(scene_device &s, cudaStream_t st);
 int kernels_per_substep(const scene_device &s);
+// activation and binning in one launch (where fused_prepare says so)
+bool fused_prepare(const scene_device &s);
+cudaError_t launch_prepare(scene_device &s, bool activate, bool bin, cudaStream_t st);
 // the implicit system (ImplicitMPM.hpp) over node-major dof vectors [nb * 512 * 3]; a kernel
 // returns at once when `skip` (device, may be null) holds a nonzero value
 cudaError_t launch_g2p2g(scene_device &s, const float *v, float *f, long long ndofs, float dt, const int *skip,

@@ -548,6 +548,7 @@ __device__ __forceinline__ void do_bin_count(const scene_device &s) {
   }
 }
 __global__ void __launch_bounds__(kThreads) k_bin_count(scene_device s) {
+  // (k_prepare, where the movers are counted beside this, has it from do_begin)
   if (blockIdx.x == 0 && threadIdx.x == 0) s.ctr[kCtrDirty] = 0;
   do_bin_count(s);
 }
@@ -864,6 +865,206 @@ __global__ void __launch_bounds__(kThreads) k_inc_finalize(scene_device s) {
 #pragma unroll
     for (int ch = 0; ch < kGridChannels; ++ch) s.grid[((size_t)b * kGridChannels + ch) * 512 + cell] = 0.f;
     if (cell == 0) s.block_count[b] = 0;
+  }
+}
+
+// ----------------------------------------------------------------- activation and binning in one launch
+// The same passes as above in one cooperative kernel, with grid barriers in place of the kernel
+// boundaries: eight of them instead of 25 launches.  Scans over few entries (the bitmap's words,
+// the blocks) are done by every CTA for itself.  A launch boundary costs about 2.5 us here, a
+// barrier about 1 us, so this is the path wherever the passes are short (fused_prepare).
+constexpr int kPrepThreads = 512;
+constexpr int kPrepScan = 4096;  // entries a CTA scans by itself
+
+// All CTAs of the (cooperative) grid arrive; false when the wait gave up (kStatusTimeout is set and the
+// caller leaves).  `target` counts the arrivals up to and with this barrier.
+__device__ __forceinline__ bool prep_barrier(const scene_device &s, int &target, int *ok) {
+  target += gridDim.x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&s.ctr[kCtrBarrier], 1);
+    int seen = 0;
+    for (int i = 0; i < (1 << 21); ++i) {
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(&s.ctr[kCtrBarrier]) : "memory");
+      if (seen >= target) break;
+    }
+    __threadfence();
+    *ok = seen >= target;
+    if (seen < target) set_status(s.ctr, kStatusTimeout);
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+// Exclusive scan of load(0 .. n) by this CTA into out[0 .. n] (shared memory, n <= kPrepScan)
+template <class Load>
+__device__ __forceinline__ void prep_scan_local(Load load, int n, int *out, int *sm) {
+  const int per = (n + kPrepThreads - 1) / kPrepThreads, lo = min(n, (int)threadIdx.x * per), hi = min(n, lo + per);
+  int sum = 0;
+  for (int i = lo; i < hi; ++i) sum += load(i);
+  int total, run = cta_exclusive_scan<kPrepThreads>(sum, total, sm);
+  for (int i = lo; i < hi; ++i) {
+    out[i] = run;
+    run += load(i);
+  }
+  if (threadIdx.x == 0) out[n] = total;
+  __syncthreads();
+}
+
+// The same over many entries, with the whole grid, into out[0 .. n] in global memory (two barriers)
+template <class Load>
+__device__ __forceinline__ bool prep_scan_grid(const scene_device &s, Load load, int n, int *out, int *sm, int &target,
+                                               int *ok) {
+  const int chunk = (n + gridDim.x - 1) / gridDim.x;
+  const int lo = min(n, (int)blockIdx.x * chunk), hi = min(n, lo + chunk);
+  int acc = 0, total;
+  for (int i = lo + threadIdx.x; i < hi; i += kPrepThreads) acc += load(i);
+  cta_exclusive_scan<kPrepThreads>(acc, total, sm);
+  if (threadIdx.x == 0) s.scan_part[blockIdx.x] = total;
+  if (!prep_barrier(s, target, ok)) return false;
+  int before = 0, run;
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += kPrepThreads) before += s.scan_part[i];
+  cta_exclusive_scan<kPrepThreads>(before, run, sm);
+  for (int base = lo; base < hi; base += kPrepThreads) {
+    const int i = base + threadIdx.x;
+    const int ex = cta_exclusive_scan<kPrepThreads>(i < hi ? load(i) : 0, total, sm);
+    if (i < hi) out[i] = run + ex;
+    run += total;
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = run;
+  return prep_barrier(s, target, ok);
+}
+
+// cell starts, a warp per block (16 consecutive cells a lane), and the work order
+__device__ __forceinline__ void prep_cell_start(const scene_device &s, int nb, const int *block_start) {
+  const int lane = threadIdx.x & 31;
+  for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += grid_threads() >> 5) {
+    const int4 *in = reinterpret_cast<const int4 *>(s.cell_count + (size_t)b * 512) + 4 * lane;
+    int c[16];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int4 v = in[q];
+      c[4 * q] = v.x, c[4 * q + 1] = v.y, c[4 * q + 2] = v.z, c[4 * q + 3] = v.w;
+    }
+    int sum = 0;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const int n = (c[q] & 0xffff) + (c[q] >> 16);  // counted in place + arrivals (k_cell_start)
+      c[q] = sum;
+      sum += n;
+    }
+    int x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, x, o);
+      if (lane >= o) x += y;
+    }
+    const int total = __shfl_sync(kFull, x, 31), base = block_start[b] + x - sum;
+    int4 *out = reinterpret_cast<int4 *>(s.cell_start + (size_t)b * 512) + 4 * lane;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      out[q] = make_int4(base + c[4 * q], base + c[4 * q + 1], base + c[4 * q + 2], base + c[4 * q + 3]);
+    if (lane == 0) {
+      s.bmask[b] = 0u;  // (G2P's items add to it)
+      if (total >= kBigBlock)
+        s.work_order[atomicAdd(&s.ctr[kCtrOrderFront], 1)] = b;
+      else if (total > 0)
+        s.work_order[nb - 1 - atomicAdd(&s.ctr[kCtrOrderBack], 1)] = b;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kPrepThreads, 2) k_prepare(scene_device s, int activate, int bin) {
+  __shared__ int sm[kPrepThreads / 32 + 1];
+  __shared__ int s_ok;
+  __shared__ int s_scan[kPrepScan + 1];
+  int target = 0;
+  // (a wait that gives up leaves through the end, where the barrier counters are cleared)
+  do {
+    if (activate) {
+      do_begin(s);
+      if (!prep_barrier(s, target, &s_ok)) break;
+      do_insert_particle_blocks(s);
+      do_insert_moved_blocks(s);
+      if (!prep_barrier(s, target, &s_ok)) break;
+      do_enlarge(s);
+      if (!prep_barrier(s, target, &s_ok)) break;
+      int nb, words;
+      block_totals(s, blockIdx.x == 0 && threadIdx.x == 0, nb, words);
+      do_bitmap_set(s, words > 0 ? nb : 0);
+      if (!prep_barrier(s, target, &s_ok)) break;
+      const load_popc popc{s.bitmap};
+      if (words <= kPrepScan) {
+        prep_scan_local(popc, words, s_scan, sm);
+        do_assign_ranks(s, words > 0 ? nb : 0, s_scan);
+      } else {
+        if (!prep_scan_grid(s, popc, words, s.word_prefix, sm, target, &s_ok)) break;
+        do_assign_ranks(s, nb, s.word_prefix);
+      }
+      if (!prep_barrier(s, target, &s_ok)) break;
+      do_neighbors(s);
+    }
+    if (bin) {
+      // (the neighbours above and the counts below both only need the ranks)
+      do_bin_count(s);
+      do_inc_stayers<true>(s);
+      do_inc_movers(s);
+      if (!prep_barrier(s, target, &s_ok)) break;
+      const int nb = s.ctr[kCtrBlocks];
+      const load_int count{s.block_count};
+      if (nb < kPrepScan) {
+        prep_scan_local(count, nb, s_scan, sm);
+        if (blockIdx.x == 0)
+          for (int i = threadIdx.x; i <= nb; i += kPrepThreads) s.block_start[i] = s_scan[i];
+        prep_cell_start(s, nb, s_scan);
+      } else {
+        if (!prep_scan_grid(s, count, nb, s.block_start, sm, target, &s_ok)) break;
+        prep_cell_start(s, nb, s.block_start);
+      }
+      if (!prep_barrier(s, target, &s_ok)) break;
+      const bool inc = incremental_binning(s);
+      do_bin_scatter(s);
+      do_inc_place_stayers(s);
+      do_inc_place_movers(s);
+      // the grid starts zeroed
+      const long long quads = (long long)nb * (kGridChannels * 512 / 4);
+      for (long long q = blockIdx.x * (long long)kPrepThreads + threadIdx.x; q < quads; q += grid_threads())
+        reinterpret_cast<float4 *>(s.grid)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!prep_barrier(s, target, &s_ok)) break;
+      // the cells' lists by upload id (incremental: those that received movers), and the counts
+      // zeroed for the next binning; a cell's length from the starts
+      auto cell_len = [&](int j) {
+        return ((j & 511) < 511 ? s.cell_start[j + 1] : s.block_start[(j >> 9) + 1]) - s.cell_start[j];
+      };
+      const int t0 = blockIdx.x * kPrepThreads + threadIdx.x;
+      if (inc) {
+        const int nd = min(s.ctr[kCtrDirty], s.prm.mover_cap);
+        for (int k = t0; k < nd; k += grid_threads()) {
+          const int j = s.dirty[k], c = cell_len(j);
+          if (c > 1) sort_cell_by_id(s, s.src, s.src, s.cell_start[j], c);
+        }
+      }
+      const long long cells = (long long)nb * 512;
+      for (long long j = t0; j < cells; j += grid_threads()) {
+        if (!inc) sort_cell_by_id(s, s.tmp, s.src, s.cell_start[j], cell_len((int)j));
+        s.cell_count[j] = 0;
+        if ((j & 511) == 0) s.block_count[j >> 9] = 0;
+      }
+      if (t0 == 0) {
+        s.ctr[kCtrBinInfo] = inc ? min(s.ctr[kCtrMovers], s.prm.mover_cap) : -1;
+        s.ctr[kCtrMovers] = 0;  // the next G2P lists its movers afresh
+      }
+    }
+  } while (false);
+  // the last CTA to leave clears the barrier for the next launch
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&s.ctr[kCtrBarrierExit], 1) == (int)gridDim.x - 1) {
+      s.ctr[kCtrBarrier] = 0;
+      s.ctr[kCtrBarrierExit] = 0;
+    }
   }
 }
 
@@ -2715,7 +2916,32 @@ int num_sms() {
 }  // namespace
 
 // ----------------------------------------------------------------- launchers
+// Whether activation and binning run as one cooperative launch (k_prepare): where the particles are few
+// enough that the passes cost less than the launches' boundaries.
+// Measured, substep with and without it: 4 k particles 0.071 / 0.091 ms, 140 k 0.095 / 0.109, 490 k
+// 0.167 / 0.171, 3.7 M 0.515 / 0.510, 16 M 2.06 / 1.98.  With a learned closure the closure pass
+// runs beside activation and binning, and a cooperative grid waits for room beside it (3.7 M:
+// 1.09 / 1.03 ms), so those scenes keep the launches.
+constexpr int kPrepMaxParticles = 1 << 20;
+bool fused_prepare(const scene_device &s) { return s.prm.cap <= kPrepMaxParticles && !s.aux.learned; }
+
+cudaError_t launch_prepare(scene_device &s, bool activate, bool bin, cudaStream_t st) {
+  const int sm = num_sms();
+  cudaLaunchConfig_t cfg = {};
+  // about four particles a thread, at most two CTAs per SM (all CTAs are resident at once)
+  cfg.gridDim = dim3((unsigned)std::min(2 * sm, std::max(64, s.prm.n / (4 * kPrepThreads))));
+  cfg.blockDim = dim3(kPrepThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_prepare, s, activate ? 1 : 0, bin ? 1 : 0);
+}
+
 cudaError_t launch_activate(scene_device &s, cudaStream_t st) {
+  if (fused_prepare(s)) return launch_prepare(s, true, false, st);
   const int sm = num_sms();
   k_begin<<<sm * 4, kThreads, 0, st>>>(s);
   k_insert_particle_blocks<<<sm * 16, kThreads, 0, st>>>(s);
@@ -2733,6 +2959,7 @@ cudaError_t launch_activate(scene_device &s, cudaStream_t st) {
 // Both binnings are enqueued; each kernel returns at once unless the device counter
 // kCtrIncBin (set by the activation) selects its path, so one CUDA graph serves both.
 cudaError_t launch_bin(scene_device &s, cudaStream_t st) {
+  if (fused_prepare(s)) return launch_prepare(s, false, true, st);
   const int sm = num_sms();
   k_bin_count<<<sm * 16, kThreads, 0, st>>>(s);
   k_inc_map<<<sm, kThreads, 0, st>>>(s);
@@ -2940,10 +3167,10 @@ cudaError_t launch_cg_iteration(scene_device &s, float *x, const cg_vectors &v, 
   return cudaGetLastError();
 }
 
-// k_begin, the two particle-block inserts (one returns at once), enlarge, prepare, set,
+// k_prepare, or: k_begin, the two particle-block inserts (one returns at once), enlarge, prepare, set,
 // 3 scans, ranks, neighbours; the binning's 14 launches (the full and the incremental path, one of
 // which returns at once).  Then p2g; grid update and boundaries; g2p
-int kernels_per_substep(const scene_device &) { return 11 + 14 + 4; }
+int kernels_per_substep(const scene_device &s) { return (fused_prepare(s) ? 1 : 11 + 14) + 4; }
 
 cudaError_t launch_import(scene_device &s, const float *m, const float *x, const float *v,
                           const float *C, const float *F, const float *plastic, int n,
