@@ -45,7 +45,6 @@ struct zsmpm_closure {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kTile = 32;  // samples per CTA in training
 
 __device__ __forceinline__ uint64_t mix64(uint64_t x) {
   x += 0x9E3779B97F4A7C15ull;
@@ -222,136 +221,317 @@ __global__ void k_closure_stats(const float *x, const float *r, const float *y, 
 }
 
 __device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float silu_grad(float z) {
-  const float s = 1.f / (1.f + expf(-z));
-  return s * (1.f + z * (1.f - s));
-}
 
 struct norm_dev {
   float in_mean[6], in_inv_std[6], out_inv_scale[6];
 };
 
-// Shared-memory copy of the weights with each row padded by one float (row stride kin + 1), so
-// that threads of a warp reading W[j][k] for consecutive j hit distinct banks.
-constexpr int kSW1 = 0, kSB1 = kSW1 + 64 * 7, kSW2 = kSB1 + 64, kSB2 = kSW2 + 64 * 65, kSW3 = kSB2 + 64,
-              kSB3 = kSW3 + 64 * 65, kSW4 = kSB3 + 64, kSB4 = kSW4 + 6 * 65, kSParams = kSB4 + 8;
+// Forward + backward of the MSE loss on normalised data: gradients (mean over `total` samples) are
+// added to grad, and the loss to *loss.  Sample k of the batch (k < count) is data row
+// ((first + k) * stride) % n_data.  kRaw: x and y are raw rows (closure_inputs and
+// closure_net_targets are applied here), else network inputs and targets.
+//
+// A CTA of 256 threads takes tiles of 16 SPT samples and keeps its gradients in registers over all of
+// them, so the 9,158 sums go to memory once per CTA (with a CTA per 32 samples and an atomic
+// per gradient entry each, 64 k samples made 18.8 M atomics on 9,158 addresses: 0.9 ms).  The
+// products are FP32 register tiles: SPT samples x 4 outputs a thread forwards and for the
+// inputs' gradients, 4 x 4 for the weights'.  Activations lie feature-major (rows of samples) in
+// shared memory, which serves all three products with 16-byte loads; the activations'
+// derivatives stay in the registers of the thread that needs them on the way back.  Bound by
+// FMA issue and shared-memory loads (26.7 k FMA a sample).
+// SPT = 8 where the tiles fill the chip, 4 for small batches.
+constexpr int kTrainRow2 = 68;  // padded weight rows
+template <int SPT>
+struct train_shape {
+  static constexpr int kTileS = 16 * SPT, kRow = kTileS + 4;  // padded sample rows
+  static constexpr int kW1 = 0, kW2 = kW1 + 64 * 8, kW3 = kW2 + 64 * kTrainRow2, kW4 = kW3 + 64 * kTrainRow2,
+                       kB = kW4 + 6 * kTrainRow2, kX = kB + 200, kD = kX + 6 * kRow, kA1 = kD + 6 * kRow,
+                       kA2 = kA1 + 64 * kRow, kA3 = kA2 + 64 * kRow, kZ = kA3 + 64 * kRow, kFloats = kZ + 64 * kRow;
+};
 
-__device__ __forceinline__ void load_padded(const float *p, float *W) {
-  for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) {
-    int dst;
-    if (i < kOffB1) dst = kSW1 + (i / 6) * 7 + i % 6;
-    else if (i < kOffW2) dst = kSB1 + (i - kOffB1);
-    else if (i < kOffB2) dst = kSW2 + ((i - kOffW2) / 64) * 65 + (i - kOffW2) % 64;
-    else if (i < kOffW3) dst = kSB2 + (i - kOffB2);
-    else if (i < kOffB3) dst = kSW3 + ((i - kOffW3) / 64) * 65 + (i - kOffW3) % 64;
-    else if (i < kOffW4) dst = kSB3 + (i - kOffB3);
-    else if (i < kOffB4) dst = kSW4 + ((i - kOffW4) / 64) * 65 + (i - kOffW4) % 64;
-    else dst = kSB4 + (i - kOffB4);
-    W[dst] = p[i];
+template <int SPT, bool kRaw>
+__global__ void __launch_bounds__(kThreads, 1) k_mlp_train(closure_dev cd, const float *__restrict__ params,
+                                                           const float *__restrict__ x, const float *__restrict__ y,
+                                                           int64_t n_data, int64_t first, int64_t count,
+                                                           int64_t stride, int64_t total, norm_dev nd, float *grad,
+                                                           float *loss) {
+  using sh = train_shape<SPT>;
+  constexpr int T = sh::kTileS, R = sh::kRow, V = SPT / 4;  // V: 16-byte vectors of samples a thread holds
+  extern __shared__ __align__(16) float smem[];
+  float *const W1 = smem + sh::kW1, *const W2 = smem + sh::kW2, *const W3 = smem + sh::kW3, *const W4 = smem + sh::kW4;
+  float *const bias = smem + sh::kB, *const X = smem + sh::kX, *const D = smem + sh::kD;
+  float *const A1 = smem + sh::kA1, *const A2 = smem + sh::kA2, *const A3 = smem + sh::kA3, *const Z = smem + sh::kZ;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int i = t; i < 64 * 6; i += kThreads) W1[i / 6 * 8 + i % 6] = params[kOffW1 + i];
+  for (int i = t; i < 64 * 64; i += kThreads) {
+    W2[i / 64 * kTrainRow2 + i % 64] = params[kOffW2 + i];
+    W3[i / 64 * kTrainRow2 + i % 64] = params[kOffW3 + i];
   }
-}
+  for (int i = t; i < 6 * 64; i += kThreads) W4[i / 64 * kTrainRow2 + i % 64] = params[kOffW4 + i];
+  if (t < 64) {
+    bias[t] = params[kOffB1 + t];
+    bias[64 + t] = params[kOffB2 + t];
+    bias[128 + t] = params[kOffB3 + t];
+    if (t < 6) bias[192 + t] = params[kOffB4 + t];
+  }
+  // samples s0 + 64 v + {0..3} (v < V), features j0 .. j0 + 3
+  const int sg = (warp & 1) * 8 + (lane & 7), s0 = 4 * sg, j0 = 4 * ((warp >> 1) * 4 + (lane >> 3));
+  // weight gradients: rows gj + 16 i, columns gk + 16 i
+  const int gk = (warp & 1) * 8 + (lane & 7), gj = (warp >> 1) * 4 + (lane >> 3);
+  float g2[4][4] = {}, g3[4][4] = {}, g1[6] = {}, g4[6] = {}, gb[3][4] = {}, gb4[3] = {};
+  float lsum = 0.f;
+  const float inv = 1.f / ((float)total * 6.f);
+  const int64_t tiles = (count + T - 1) / T;
 
-// Forward + backward of the MSE loss on normalised data for one tile of 32 samples per CTA;
-// gradients (mean over `total` samples) are accumulated with atomics into grad, and the loss
-// into *loss.  Sample k of the batch (k < count) is data row ((first + k) * stride) % n_data.
-__global__ void __launch_bounds__(kThreads) k_mlp_train_tile(const float *params, const float *x, const float *y,
-                                                             int64_t n_data, int64_t first, int64_t count,
-                                                             int64_t stride, int64_t total, norm_dev nd,
-                                                             float *grad, float *loss) {
-  extern __shared__ float smem[];
-  float *W = smem;                                  // kSParams (padded rows)
-  float *A0 = W + kSParams;                         // [32][6]
-  float *Z1 = A0 + kTile * 6, *A1 = Z1 + kTile * 64;
-  float *Z2 = A1 + kTile * 64, *A2 = Z2 + kTile * 64;
-  float *Z3 = A2 + kTile * 64, *A3 = Z3 + kTile * 64;
-  float *OUT = A3 + kTile * 64;                     // [32][6]
-  float *Y = OUT + kTile * 6;                       // [32][6]
-  float *dA = Y + kTile * 6;                        // [32][64]
-  float *dZ = dA + kTile * 64;                      // [32][64]
-  const int t = threadIdx.x;
-  const int64_t base = (int64_t)blockIdx.x * kTile;
-  load_padded(params, W);
-  for (int i = t; i < kTile * 6; i += blockDim.x) {
-    const int s = i / 6, k = i % 6;
-    const int64_t row = base + s;
-    float xv = 0.f, yv = 0.f;
-    if (row < count) {
-      const int64_t r = (int64_t)(((unsigned long long)(first + row) * (unsigned long long)stride) %
-                                  (unsigned long long)n_data);
-      xv = (x[6 * r + k] - nd.in_mean[k]) * nd.in_inv_std[k];
-      yv = y[6 * r + k] * nd.out_inv_scale[k];
+  // z(s, j) = b(j) + sum_k in(k, s) W(j, k); activations to `out`, derivatives to d
+  auto activate = [&](float (&acc)[4][SPT], float *out, float (&d)[4][SPT]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+      for (int q = 0; q < SPT; ++q) {
+        const float z = acc[j][q];
+        // sigmoid: one reciprocal with a Newton step (the clamp keeps exp finite)
+        const float e = 1.f + expf(fminf(-z, 80.f));
+        float r = __fdividef(1.f, e);
+        r = fmaf(fmaf(-e, r, 1.f), r, r);
+        acc[j][q] = z * r;
+        d[j][q] = r * fmaf(z, 1.f - r, 1.f);
+      }
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        *reinterpret_cast<float4 *>(out + (j0 + j) * R + s0 + 64 * v) =
+            make_float4(acc[j][4 * v], acc[j][4 * v + 1], acc[j][4 * v + 2], acc[j][4 * v + 3]);
     }
-    A0[i] = xv;
-    Y[i] = yv;
-  }
-  __syncthreads();
-  const int valid = (int)(count - base < kTile ? count - base : kTile);
-  auto dense = [&](const float *in, int kin, const float *Wl, const float *bl, float *z, float *a, int nout,
-                   bool act) {
-    for (int i = t; i < kTile * nout; i += blockDim.x) {
-      const int s = i / nout, j = i % nout;
-      float acc = bl[j];
-      for (int k = 0; k < kin; ++k) acc += in[s * kin + k] * Wl[j * (kin + 1) + k];
-      z[i] = acc;
-      if (a) a[i] = act ? silu(acc) : acc;
+  };
+  auto load_s = [&](const float *row, float (&a)[SPT]) {
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const float4 q = *reinterpret_cast<const float4 *>(row + s0 + 64 * v);
+      a[4 * v] = q.x, a[4 * v + 1] = q.y, a[4 * v + 2] = q.z, a[4 * v + 3] = q.w;
+    }
+  };
+  auto forward = [&](const float *in, const float *W, const float *b, float *out, float (&d)[4][SPT]) {
+    float acc[4][SPT];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int q = 0; q < SPT; ++q) acc[j][q] = b[j0 + j];
+#pragma unroll 2
+    for (int k = 0; k < 64; k += 4) {
+      float4 w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4 *>(W + (j0 + j) * kTrainRow2 + k);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float a[SPT];
+        load_s(in + (k + u) * R, a);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float wj = u == 0 ? w[j].x : u == 1 ? w[j].y : u == 2 ? w[j].z : w[j].w;
+#pragma unroll
+          for (int q = 0; q < SPT; ++q) acc[j][q] = fmaf(a[q], wj, acc[j][q]);
+        }
+      }
+    }
+    activate(acc, out, d);
+  };
+  // din(k, s) = sum_j dz(j, s) W(j, k) over NJ rows, times the derivative: the next dz, in registers
+  auto back_input = [&](const float *dz, int nj, const float *W, float (&d)[4][SPT]) {
+    float acc[4][SPT] = {};
+#pragma unroll 4
+    for (int j = 0; j < nj; ++j) {
+      const float4 w = *reinterpret_cast<const float4 *>(W + j * kTrainRow2 + j0);
+      float a[SPT];
+      load_s(dz + j * R, a);
+#pragma unroll
+      for (int q = 0; q < SPT; ++q) {
+        acc[0][q] = fmaf(a[q], w.x, acc[0][q]);
+        acc[1][q] = fmaf(a[q], w.y, acc[1][q]);
+        acc[2][q] = fmaf(a[q], w.z, acc[2][q]);
+        acc[3][q] = fmaf(a[q], w.w, acc[3][q]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int q = 0; q < SPT; ++q) d[j][q] *= acc[j][q];
+  };
+  auto store_dz = [&](const float (&d)[4][SPT], float (&b)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float sum = 0.f;
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        *reinterpret_cast<float4 *>(Z + (j0 + j) * R + s0 + 64 * v) =
+            make_float4(d[j][4 * v], d[j][4 * v + 1], d[j][4 * v + 2], d[j][4 * v + 3]);
+        sum += (d[j][4 * v] + d[j][4 * v + 1]) + (d[j][4 * v + 2] + d[j][4 * v + 3]);
+      }
+      b[j] += sum;
+    }
+  };
+  // g(j, k) += sum_s dz(j, s) a(k, s)
+  auto back_weights = [&](const float *a, float (&g)[4][4]) {
+#pragma unroll 2
+    for (int s = 0; s < T; s += 4) {
+      float4 p[4], q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        p[i] = *reinterpret_cast<const float4 *>(Z + (gj + 16 * i) * R + s);
+        q[i] = *reinterpret_cast<const float4 *>(a + (gk + 16 * i) * R + s);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          g[i][k] = fmaf(p[i].x, q[k].x, fmaf(p[i].y, q[k].y, fmaf(p[i].z, q[k].z, fmaf(p[i].w, q[k].w, g[i][k]))));
+    }
+  };
+  // six sums over a quarter of the tile's samples: rows `six` against feature row t & 63 of `a`
+  auto back_six = [&](const float *six, const float *a, float (&g)[6]) {
+    const float *row = a + (t & 63) * R;
+#pragma unroll 2
+    for (int s = (t >> 6) * (T / 4); s < ((t >> 6) + 1) * (T / 4); s += 4) {
+      const float4 p = *reinterpret_cast<const float4 *>(row + s);
+#pragma unroll
+      for (int o = 0; o < 6; ++o) {
+        const float4 q = *reinterpret_cast<const float4 *>(six + o * R + s);
+        g[o] = fmaf(p.x, q.x, fmaf(p.y, q.y, fmaf(p.z, q.z, fmaf(p.w, q.w, g[o]))));
+      }
+    }
+  };
+
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    __syncthreads();  // weights in place; the last tile's arrays are free
+    if (t < T) {
+      const int64_t row = tile * T + t;
+      float in[6] = {}, tg[6] = {};
+      if (row < count) {
+        const int64_t r = (int64_t)(((unsigned long long)(first + row) * (unsigned long long)stride) %
+                                    (unsigned long long)n_data);
+        float xr[6], yr[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          xr[k] = x[6 * r + k];
+          yr[k] = y[6 * r + k];
+        }
+        if (kRaw) {
+          net_scale ns;
+          closure_inputs(cd.model, cd.kappa, cd.hardening, xr, in, ns);
+          closure_net_targets(ns, yr, tg);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 6; ++k) {
+            in[k] = xr[k];
+            tg[k] = yr[k];
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          in[k] = (in[k] - nd.in_mean[k]) * nd.in_inv_std[k];
+          tg[k] *= nd.out_inv_scale[k];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        X[k * R + t] = in[k];
+        D[k * R + t] = tg[k];
+      }
     }
     __syncthreads();
-  };
-  dense(A0, 6, W + kSW1, W + kSB1, Z1, A1, 64, true);
-  dense(A1, 64, W + kSW2, W + kSB2, Z2, A2, 64, true);
-  dense(A2, 64, W + kSW3, W + kSB3, Z3, A3, 64, true);
-  dense(A3, 64, W + kSW4, W + kSB4, OUT, nullptr, 6, false);
-  // dL/dOUT for L = mean over samples and outputs of (OUT - Y)^2
-  const float inv = 1.f / ((float)total * 6.f);
-  float lsum = 0.f;
-  for (int i = t; i < kTile * 6; i += blockDim.x) {
-    const int s = i / 6;
-    const float e = s < valid ? OUT[i] - Y[i] : 0.f;
-    dZ[i] = 2.f * e * inv;  // dOUT stored in dZ[32][6]
-    lsum += e * e * inv;
+    float d1[4][SPT], d2[4][SPT], d3[4][SPT];
+    {
+      float acc[4][SPT];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int q = 0; q < SPT; ++q) acc[j][q] = bias[j0 + j];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        float a[SPT];
+        load_s(X + k * R, a);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float w = W1[(j0 + j) * 8 + k];
+#pragma unroll
+          for (int q = 0; q < SPT; ++q) acc[j][q] = fmaf(a[q], w, acc[j][q]);
+        }
+      }
+      activate(acc, A1, d1);
+    }
+    __syncthreads();
+    forward(A1, W2, bias + 64, A2, d2);
+    __syncthreads();
+    forward(A2, W3, bias + 128, A3, d3);
+    __syncthreads();
+    // outputs, their error and its gradient: thread (sample, three outputs)
+    if (t < 2 * T) {
+      const int s = t & (T - 1), o0 = t / T * 3;
+      float out[3] = {bias[192 + o0], bias[193 + o0], bias[194 + o0]};
+#pragma unroll 4
+      for (int k = 0; k < 64; ++k) {
+        const float a = A3[k * R + s];
+#pragma unroll
+        for (int o = 0; o < 3; ++o) out[o] = fmaf(a, W4[(o0 + o) * kTrainRow2 + k], out[o]);
+      }
+      const bool valid = tile * T + s < count;
+#pragma unroll
+      for (int o = 0; o < 3; ++o) {
+        float *const at = D + (o0 + o) * R + s;
+        const float e = valid ? out[o] - *at : 0.f, de = 2.f * e * inv;
+        *at = de;
+        lsum += e * e * inv;
+        gb4[o] += de;
+      }
+    }
+    __syncthreads();
+    back_six(D, A3, g4);
+    back_input(D, 6, W4, d3);  // d3 is now dz of layer 3
+    store_dz(d3, gb[2]);
+    __syncthreads();
+    back_weights(A2, g3);
+    back_input(Z, 64, W3, d2);
+    __syncthreads();
+    store_dz(d2, gb[1]);
+    __syncthreads();
+    back_weights(A1, g2);
+    back_input(Z, 64, W2, d1);
+    __syncthreads();
+    store_dz(d1, gb[0]);
+    __syncthreads();
+    back_six(X, Z, g1);
+  }
+  // this CTA's sums
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      atomicAdd(&grad[kOffW2 + (gj + 16 * i) * 64 + gk + 16 * k], g2[i][k]);
+      atomicAdd(&grad[kOffW3 + (gj + 16 * i) * 64 + gk + 16 * k], g3[i][k]);
+    }
+#pragma unroll
+  for (int o = 0; o < 6; ++o) {
+    atomicAdd(&grad[kOffW1 + (t & 63) * 6 + o], g1[o]);
+    atomicAdd(&grad[kOffW4 + o * 64 + (t & 63)], g4[o]);
+  }
+  // the biases: over the eight lanes of a feature group, then by atomics
+#pragma unroll
+  for (int l = 0; l < 3; ++l)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float v = gb[l][j];
+      for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if ((lane & 7) == 0) atomicAdd(&grad[(l == 0 ? kOffB1 : l == 1 ? kOffB2 : kOffB3) + j0 + j], v);
+    }
+  const int o0 = t / T * 3;  // (uniform over a warp)
+#pragma unroll
+  for (int o = 0; o < 3; ++o) {
+    float v = gb4[o];
+    for (int q = 16; q > 0; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
+    if (lane == 0 && t < 2 * T) atomicAdd(&grad[kOffB4 + o0 + o], v);
   }
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if ((t & 31) == 0) atomicAdd(loss, lsum);
-  __syncthreads();
-  // back through a dense layer: gW[j][k] += sum_s dz[s][j] in[s][k]; gb[j] += sum_s dz[s][j];
-  // din[s][k] = sum_j dz[s][j] W[j][k]
-  auto back = [&](const float *dz, int nout, const float *in, int kin, const float *Wl, float *gW, float *gb,
-                  float *din) {
-    for (int i = t; i < nout * kin; i += blockDim.x) {
-      const int j = i / kin, k = i % kin;
-      float acc = 0.f;
-      for (int s = 0; s < kTile; ++s) acc += dz[s * nout + j] * in[s * kin + k];
-      atomicAdd(&gW[i], acc);
-    }
-    for (int j = t; j < nout; j += blockDim.x) {
-      float acc = 0.f;
-      for (int s = 0; s < kTile; ++s) acc += dz[s * nout + j];
-      atomicAdd(&gb[j], acc);
-    }
-    if (din)
-      for (int i = t; i < kTile * kin; i += blockDim.x) {
-        const int s = i / kin, k = i % kin;
-        float acc = 0.f;
-        for (int j = 0; j < nout; ++j) acc += dz[s * nout + j] * Wl[j * (kin + 1) + k];
-        din[i] = acc;
-      }
-    __syncthreads();
-  };
-  auto through_silu = [&](const float *da, const float *z, float *dz) {
-    for (int i = t; i < kTile * 64; i += blockDim.x) dz[i] = da[i] * silu_grad(z[i]);
-    __syncthreads();
-  };
-  back(dZ, 6, A3, 64, W + kSW4, grad + kOffW4, grad + kOffB4, dA);
-  through_silu(dA, Z3, dZ);
-  back(dZ, 64, A2, 64, W + kSW3, grad + kOffW3, grad + kOffB3, dA);
-  through_silu(dA, Z2, dZ);
-  back(dZ, 64, A1, 64, W + kSW2, grad + kOffW2, grad + kOffB2, dA);
-  through_silu(dA, Z1, dZ);
-  back(dZ, 64, A0, 6, W + kOffW1, grad + kOffW1, grad + kOffB1, nullptr);
+  if (lane == 0) atomicAdd(loss, lsum);
 }
-
-constexpr size_t kTrainSmem =
-    sizeof(float) * (kSParams + kTile * 6 + 6 * kTile * 64 + kTile * 6 * 2 + 2 * kTile * 64);
 
 __global__ void k_adam(float *p, float *g, float *m, float *v, int n, float lr, float b1, float b2,
                        float eps, float c1, float c2) {
@@ -776,17 +956,41 @@ int sms() {
   return n > 0 ? n : 148;
 }
 
-// the training kernel's shared-memory size (above the 48 KB default), once per device
+// the training kernels' shared-memory sizes (above the 48 KB default), once per device
 cudaError_t prepare_train_kernel(int device) {
   static std::mutex mu;
   static std::vector<char> done;
   std::lock_guard<std::mutex> lock(mu);
   if ((int)done.size() <= device) done.resize(device + 1, 0);
   if (done[device]) return cudaSuccess;
-  const cudaError_t e =
-      cudaFuncSetAttribute(k_mlp_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem);
+  cudaError_t e = cudaSuccess;
+  auto size = [&](const void *fn, int floats) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, floats * (int)sizeof(float));
+  };
+  size((const void *)k_mlp_train<8, false>, train_shape<8>::kFloats);
+  size((const void *)k_mlp_train<8, true>, train_shape<8>::kFloats);
+  size((const void *)k_mlp_train<4, false>, train_shape<4>::kFloats);
+  size((const void *)k_mlp_train<4, true>, train_shape<4>::kFloats);
   if (e == cudaSuccess) done[device] = 1;
   return e;
+}
+
+// loss and gradients of a batch; tiles of 64 samples unless tiles of 128 fill the chip
+template <bool kRaw>
+void launch_train(const closure_dev &cd, const float *params, const float *x, const float *y, int64_t n_data,
+                  int64_t first, int64_t count, int64_t stride, const norm_dev &nd, float *grad, float *loss,
+                  cudaStream_t st) {
+  const int64_t sm = sms();
+  if (count >= 128 * sm) {
+    const int64_t tiles = (count + 127) / 128;
+    k_mlp_train<8, kRaw><<<(int)std::min(tiles, sm), kThreads, train_shape<8>::kFloats * sizeof(float), st>>>(
+        cd, params, x, y, n_data, first, count, stride, count, nd, grad, loss);
+  } else {
+    const int64_t tiles = (count + 63) / 64;
+    k_mlp_train<4, kRaw><<<(int)std::min(tiles, sm), kThreads, train_shape<4>::kFloats * sizeof(float), st>>>(
+        cd, params, x, y, n_data, first, count, stride, count, nd, grad, loss);
+  }
 }
 
 // deterministic Xavier-uniform initial weights, zero biases
@@ -1024,7 +1228,7 @@ ZSMPM_API zsmpm_status zsmpm_closure_dataset_size(const zsmpm_closure *c, int64_
 
 ZSMPM_API zsmpm_status zsmpm_closure_train(zsmpm_closure *c, int32_t epochs, int32_t batch, float lr, uint64_t seed,
                                            float *loss_out, void *stream) {
-  if (!c || !c->normalized || c->data_n < 1 || epochs < 1 || batch < kTile || !(lr > 0.f))
+  if (!c || !c->normalized || c->data_n < 1 || epochs < 1 || batch < 32 || !(lr > 0.f))
     return cerr(ZSMPM_ERR_INVALID_ARG, "train needs a dataset, epochs >= 1, batch >= 32, lr > 0");
   CZ_TRY(cudaSetDevice(c->device), "cudaSetDevice");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1047,9 +1251,7 @@ ZSMPM_API zsmpm_status zsmpm_closure_train(zsmpm_closure *c, int32_t epochs, int
     for (int64_t s = 0; s < steps; ++s) {
       const int64_t first = offset + s * batch;
       const int64_t count = std::min<int64_t>(batch, n - s * batch);
-      const int tiles = (int)((count + kTile - 1) / kTile);
-      k_mlp_train_tile<<<tiles, kThreads, kTrainSmem, st>>>(c->params, c->data_xt, c->data_yt, n, first, count,
-                                                            stride, count, nd, c->grad, c->loss);
+      launch_train<false>(c->cd, c->params, c->data_xt, c->data_yt, n, first, count, stride, nd, c->grad, c->loss, st);
       ++c->adam_t;
       const float b1 = 0.9f, b2 = 0.999f;
       const float c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)c->adam_t)));
@@ -1073,21 +1275,11 @@ ZSMPM_API zsmpm_status zsmpm_closure_loss_grad(zsmpm_closure *c, const float *x,
   CZ_TRY(cudaSetDevice(c->device), "cudaSetDevice");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CZ_TRY(prepare_train_kernel(c->device), "train smem");
-  float *xt = nullptr, *yt = nullptr;
-  CZ_TRY(cudaMalloc(&xt, sizeof(float) * 6 * n), "loss_grad scratch");
-  if (cudaMalloc(&yt, sizeof(float) * 6 * n) != cudaSuccess) {
-    cudaFree(xt);
-    return cerr(ZSMPM_ERR_CUDA, "loss_grad scratch");
-  }
   cudaMemsetAsync(grad, 0, sizeof(float) * kMlpParams, st);
   cudaMemsetAsync(loss, 0, sizeof(float), st);
-  k_closure_transform<<<sms() * 4, kThreads, 0, st>>>(c->cd, x, y, xt, yt, n);
-  const int tiles = (int)((n + kTile - 1) / kTile);
-  k_mlp_train_tile<<<tiles, kThreads, kTrainSmem, st>>>(c->params, xt, yt, n, 0, n, 1, n, norm_of(c->cd), grad, loss);
+  launch_train<true>(c->cd, c->params, x, y, n, 0, n, 1, norm_of(c->cd), grad, loss, st);
   const cudaError_t e = cudaGetLastError();
   const cudaError_t es = cudaStreamSynchronize(st);
-  cudaFree(xt);
-  cudaFree(yt);
   CZ_TRY(e, "loss_grad");
   CZ_TRY(es, "loss_grad sync");
   return ZSMPM_OK;
