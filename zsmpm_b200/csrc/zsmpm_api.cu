@@ -625,7 +625,6 @@ static zsmpm_status upload_arrays(zsmpm_scene *s, const zsmpm_particle_arrays *p
     if (e != cudaSuccess) return cuda_fail(e, "upload staging copy");
   }
   cudaError_t e = launch_import(s->dev, dm, dx, dv, dC, dF, dpl, (int)n, cs);
-  if (e == cudaSuccess) e = launch_prime(s->dev, cs);
   // host arrays may be reused once the call returns, and the staging buffer is free again
   if (e == cudaSuccess && !on_device) e = cudaStreamSynchronize(cs);
   if (e != cudaSuccess) return cuda_fail(e, "upload");
