@@ -1071,7 +1071,7 @@ ZSMPM_API zsmpm_status zsmpm_scene_set_closure(zsmpm_scene *s, zsmpm_closure *c,
     int *ids = nullptr;
     ZS_ALLOC(feat, 6 * q, "alloc closure queue");
     ZS_ALLOC(outr, 6 * q, "alloc closure queue");
-    ZS_ALLOC(uvs, (size_t)kQueueFloats * q, "alloc closure queue");
+    ZS_ALLOC(uvs, (size_t)kQueueFloats * mat_capacity(q), "alloc closure queue");
     ZS_ALLOC(slots, q, "alloc closure queue");
     ZS_ALLOC(ids, q, "alloc closure queue");
     s->dev.aux.q_feat = feat;

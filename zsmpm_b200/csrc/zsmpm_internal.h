@@ -119,13 +119,18 @@ constexpr int kTransferApic = 0, kTransferCell = 1;
 
 // floats of a queue entry: U 9, V 9, S 3, plastic state, m, C 9
 constexpr int kQueueFloats = 32;
+// The queue's entries lie in tiles of 32 rows, entry e of row k at queue_at(e, k), so that a warp's
+// lanes, which queue consecutive rows, touch 128 contiguous bytes per entry.
+__host__ __device__ __forceinline__ size_t queue_at(int e, size_t k) {
+  return ((k >> 5) * kQueueFloats + (size_t)e) * 32 + (k & 31);
+}
 
 // G2P options beside the plain path: the learned closure and the trial-state log.
 struct g2p_aux {
   int learned = 0;            // 1: the closure's MLP replaces the return map's projection
   closure_dev cd{};           // its weights, normalisation, hull and audit accumulators
   // the projections G2P hands to the network: raw features [qcap][6], network outputs
-  // [qcap][6], [qcap][kQueueFloats] U V S, the plastic state, m and C, (binned slot, scene)
+  // [qcap][6], U V S, the plastic state, m and C (queue_at, kQueueFloats a row), (binned slot, scene)
   // [qcap] and the upload index [qcap]
   float *q_feat = nullptr, *q_out = nullptr, *q_uvs = nullptr;
   int2 *q_slot = nullptr;

@@ -1711,21 +1711,21 @@ __device__ __forceinline__ bool learned_update(const scene_device &s, const mate
         float *fr = s.aux.q_feat + 6 * k;
 #pragma unroll
         for (int i = 0; i < 6; ++i) fr[i] = feat[i];
-        float *u = s.aux.q_uvs + kQueueFloats * k;
+        float *u = s.aux.q_uvs + queue_at(0, k);  // entry e at u[32 e]
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
-          u[i] = U[i];
-          u[9 + i] = V[i];
+          u[32 * i] = U[i];
+          u[32 * (9 + i)] = V[i];
         }
-        u[18] = S[0];
-        u[19] = S[1];
-        u[20] = S[2];
-        u[21] = plastic;
+        u[32 * 18] = S[0];
+        u[32 * 19] = S[1];
+        u[32 * 20] = S[2];
+        u[32 * 21] = plastic;
         // the particle's mass and C, for the affine momentum (so that the finish reads only the
         // queue)
-        u[22] = m;
+        u[32 * 22] = m;
 #pragma unroll
-        for (int i = 0; i < 9; ++i) u[23 + i] = Cm[i];
+        for (int i = 0; i < 9; ++i) u[32 * (23 + i)] = Cm[i];
         s.aux.q_slot[k] = make_int2(slot, sid);
         s.aux.q_id[k] = id;
         queued = true;
@@ -1783,17 +1783,17 @@ __global__ void __launch_bounds__(kThreads) k_closure_finish(scene_device s) {
     const int2 sl = s.aux.q_slot[k];
     const int slot = sl.x;
     const material_dev mat = s.prm.batch ? s.prm.mats[sl.y] : s.prm.mat;
-    const float *u = s.aux.q_uvs + kQueueFloats * (size_t)k;
+    const float *u = s.aux.q_uvs + queue_at(0, k);
     float U[9], V[9], S[3], feat[6], y[6];
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
-      U[i] = u[i];
-      V[i] = u[9 + i];
+      U[i] = u[32 * i];
+      V[i] = u[32 * (9 + i)];
     }
-    S[0] = u[18];
-    S[1] = u[19];
-    S[2] = u[20];
-    const float plastic = u[21];
+    S[0] = u[32 * 18];
+    S[1] = u[32 * 19];
+    S[2] = u[32 * 20];
+    const float plastic = u[32 * 21];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       feat[i] = s.aux.q_feat[6 * (size_t)k + i];
@@ -1842,14 +1842,14 @@ __global__ void __launch_bounds__(kThreads) k_closure_finish(scene_device s) {
     float tau[9], Fn[9];
     mul_diag_t(tau, U, dd, U);
     mul_diag_t(Fn, U, Ns, V);
-    const float m = u[22];
+    const float m = u[32 * 22];
 #pragma unroll
     for (int c = 0; c < 9; ++c) s.nxt.F[mat_at(c, slot)] = Fn[c];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {  // (the row's first entry is the velocity, which G2P wrote)
       float *const r = &s.nxt.row[row_at(d, slot)].x;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) r[1 + c] = m * u[23 + 3 * c + d] - s.prm.kappa * tau[3 * c + d];
+      for (int c = 0; c < 3; ++c) r[1 + c] = m * u[32 * (23 + 3 * c + d)] - s.prm.kappa * tau[3 * c + d];
     }
     if (s.nxt.plastic) s.nxt.plastic[slot] = pl_new;
   }
