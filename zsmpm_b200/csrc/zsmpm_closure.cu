@@ -664,8 +664,11 @@ constexpr int kTcWBytes = kTcA;                  // the packed weights
 // lo = bf16(v - hi)), each layer A_hi W_hi + A_hi W_lo + A_lo W_hi into one FP32 accumulator:
 // products to about 16 significant bits, against 8 for plain BF16 operands
 constexpr int kTcSplitA = 2 * kTcWBytes;                       // A_hi, then A_lo
-constexpr int kTcSplitSmem = kTcSplitA + 2 * kTcRows * 64 * 2;  // 72 KB: 3 CTAs per SM
-constexpr int kTcTmemCols = 64;
+#ifndef TC_GROUPS
+#define TC_GROUPS 5
+#endif
+constexpr int kTcGroups = TC_GROUPS;  // warpgroups of a CTA
+constexpr int kTcSplitSmem = kTcSplitA + kTcGroups * 2 * kTcRows * 64 * 2;  // one CTA per SM
 constexpr long long kTcWaitLimit = 1ll << 22;    // try_wait rounds before giving up
 
 __host__ __device__ constexpr int umma_offset(int R, int r, int k) {
@@ -757,6 +760,22 @@ __device__ __forceinline__ void tmem_ld64(uint32_t addr, float (&v)[64]) {
   for (int k = 0; k < 64; ++k) v[k] = __uint_as_float(r[k]);
 }
 
+// 32 columns of this thread's row of the accumulator
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, float (&v)[32]) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int k = 0; k < 32; ++k) v[k] = __uint_as_float(r[k]);
+}
+
 __device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
   uint32_t r[16];
   asm volatile(
@@ -771,31 +790,53 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
 
 // v as a hi + lo pair of bf16 (two bf16x2 words for two values)
 __device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t &hi, uint32_t &lo) {
-  const __nv_bfloat16 ha = __float2bfloat16_rn(a), hb = __float2bfloat16_rn(b);
-  hi = (uint32_t)__bfloat16_as_ushort(ha) | ((uint32_t)__bfloat16_as_ushort(hb) << 16);
-  lo = pack_bf16x2(a - __bfloat162float(ha), b - __bfloat162float(hb));
+  hi = pack_bf16x2(a, b);
+  lo = pack_bf16x2(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+}
+
+// SiLU of two values in FP32 with one reciprocal: 1/a and 1/b from 1/(ab).  The clamp keeps the
+// product finite (at z = -40 SiLU is -1.7e-16).  The epilogue is bound by the special-function
+// unit, which this takes from two to one and a half operations a value.
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void silu_pair(float za, float zb, float &a, float &b) {
+  constexpr float kLog2e = 1.4426950408889634f;
+  const float da = 1.f + exp2_ftz(fminf(za * -kLog2e, 57.7f)), db = 1.f + exp2_ftz(fminf(zb * -kLog2e, 57.7f));
+  const float r = rcp_ftz(da * db);
+  a = za * (r * db);
+  b = zb * (r * da);
 }
 
 // the split variant's epilogue: bias + SiLU in FP32, written as hi and lo rows
 __device__ __forceinline__ void tc_hidden_epilogue_split(uint32_t tmem_row, const float *bias, unsigned char *a_hi,
                                                          unsigned char *a_lo, int row) {
-  float v[64];
-  tmem_ld64(tmem_row, v);
 #pragma unroll
-  for (int kc = 0; kc < 8; ++kc) {
-    float a[8];
+  for (int half = 0; half < 2; ++half) {
+    float v[32];
+    tmem_ld32(tmem_row + 32 * half, v);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float z = v[8 * kc + j] + bias[8 * kc + j];
-      a[j] = __fdividef(z, 1.f + __expf(-z));
+    for (int kc = 0; kc < 4; ++kc) {
+      float a[8];
+#pragma unroll
+      for (int j = 0; j < 8; j += 2)
+        silu_pair(v[8 * kc + j] + bias[32 * half + 8 * kc + j], v[8 * kc + j + 1] + bias[32 * half + 8 * kc + j + 1], a[j],
+                  a[j + 1]);
+      uint4 h, l;
+      split_bf16x2(a[0], a[1], h.x, l.x);
+      split_bf16x2(a[2], a[3], h.y, l.y);
+      split_bf16x2(a[4], a[5], h.z, l.z);
+      split_bf16x2(a[6], a[7], h.w, l.w);
+      *reinterpret_cast<uint4 *>(a_hi + umma_offset(kTcRows, row, 32 * half + 8 * kc)) = h;
+      *reinterpret_cast<uint4 *>(a_lo + umma_offset(kTcRows, row, 32 * half + 8 * kc)) = l;
     }
-    uint4 h, l;
-    split_bf16x2(a[0], a[1], h.x, l.x);
-    split_bf16x2(a[2], a[3], h.y, l.y);
-    split_bf16x2(a[4], a[5], h.z, l.z);
-    split_bf16x2(a[6], a[7], h.w, l.w);
-    *reinterpret_cast<uint4 *>(a_hi + umma_offset(kTcRows, row, 8 * kc)) = h;
-    *reinterpret_cast<uint4 *>(a_lo + umma_offset(kTcRows, row, 8 * kc)) = l;
   }
 }
 
@@ -816,42 +857,60 @@ __device__ __forceinline__ void tc_hidden_epilogue(uint32_t tmem_row, const floa
   }
 }
 
+// Threads of one warpgroup (bar.sync on its own barrier)
+__device__ __forceinline__ void group_sync(int group) {
+  asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kTcRows) : "memory");
+}
+
 // n_dev (optional): the row count in device memory, at most n (the G2P queue of a substep).
 // kSplit: the split-BF16 variant (weights and activations as hi + lo BF16, three MMAs per K step).
-template <bool kSplit>
-__global__ void __launch_bounds__(kTcRows) k_closure_infer_tc(closure_dev cd, const uint4 *wpack, const float *x,
-                                                              float *y, int64_t n, const int *n_dev, int *status) {
+// A CTA of kGroups warpgroups, each with tiles, an accumulator and a completion barrier of its own;
+// they share the weights.  A tile's four layers are a serial chain (MMA, commit, wait, load,
+// epilogue), so what counts is the tiles in flight per SM: for the split variant five groups in
+// one CTA, where CTAs of one group held three (the weights again in each).  The BF16 variant's
+// CTAs are small enough for six per SM.
+template <bool kSplit, int kGroups>
+__global__ void __launch_bounds__(kTcRows *kGroups) k_closure_infer_tc(closure_dev cd, const uint4 *wpack,
+                                                                      const float *x, float *y, int64_t n,
+                                                                      const int *n_dev, int *status) {
   if (n_dev) n = min(n, (int64_t)*n_dev);
   if ((int64_t)blockIdx.x * kTcRows >= n) return;  // no tile for this CTA (before any allocation)
   extern __shared__ __align__(1024) unsigned char tsm[];
-  __shared__ __align__(8) uint64_t mbar;
+  __shared__ __align__(8) uint64_t mbar[kGroups];
   __shared__ uint32_t taddr_s;
   __shared__ float sbias[kBiasTotal];
-  const int t = threadIdx.x, warp = t >> 5;
-  for (int i = t; i < (kSplit ? 2 : 1) * kTcWBytes / 16; i += kTcRows) reinterpret_cast<uint4 *>(tsm)[i] = wpack[i];
-  for (int i = t; i < kBiasTotal; i += kTcRows) sbias[i] = cd.bias[i];
-  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&mbar);
-  if (warp == 0) {
+  __shared__ int s_fail[kGroups];
+  constexpr int kCols = kGroups <= 1 ? 64 : kGroups <= 2 ? 128 : kGroups <= 4 ? 256 : 512;  // a power of two
+  static_assert(64 * kGroups <= kCols, "tensor-memory columns");
+  const int t = threadIdx.x % kTcRows, group = threadIdx.x / kTcRows, warp = t >> 5;
+  for (int i = threadIdx.x; i < (kSplit ? 2 : 1) * kTcWBytes / 16; i += kTcRows * kGroups)
+    reinterpret_cast<uint4 *>(tsm)[i] = wpack[i];
+  for (int i = threadIdx.x; i < kBiasTotal; i += kTcRows * kGroups) sbias[i] = cd.bias[i];
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&mbar[group]);
+  if (threadIdx.x < 32) {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&taddr_s);
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(kTcTmemCols));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(kCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
-  if (t == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(1));
+  if (t == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(1));
+    s_fail[group] = 0;
+  }
   async_proxy_fence();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = taddr_s;
+  const uint32_t tmem = taddr_s + 64 * group;
   const uint32_t tmem_row = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's 32 lanes
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(tsm);
-  constexpr int a_off = kSplit ? kTcSplitA : kTcA;
+  const int a_off = (kSplit ? kTcSplitA : kTcA) + group * (kSplit ? 2 : 1) * kTcRows * 64 * 2;
   unsigned char *a_tile = tsm + a_off;  // A_hi (the only A tile without the split)
   unsigned char *a_lo = tsm + a_off + kTcRows * 64 * 2;
   const uint32_t a_addr = sbase + a_off, alo_addr = a_addr + kTcRows * 64 * 2;
   const uint32_t id64 = umma_idesc(64), id16 = umma_idesc(16);
   uint32_t parity = 0;
   bool ok = true;
-  for (int64_t tile = blockIdx.x; tile * kTcRows < n; tile += gridDim.x) {
+  for (int64_t tile = blockIdx.x + (int64_t)gridDim.x * group; tile * kTcRows < n; tile += (int64_t)gridDim.x * kGroups) {
     const int64_t row = tile * kTcRows + t;
     // input row -> network inputs -> bf16 A tile (K = 16: 6 inputs and zeros)
     float raw[6], in[kMlpIn];
@@ -883,7 +942,7 @@ __global__ void __launch_bounds__(kTcRows) k_closure_infer_tc(closure_dev cd, co
     for (int layer = 0; layer < 4 && ok; ++layer) {
       async_proxy_fence();
       tc_fence_before();
-      __syncthreads();
+      group_sync(group);
       tc_fence_after();
       if (t == 0) {
         const int ksteps = layer == 0 ? 1 : 4;
@@ -904,7 +963,9 @@ __global__ void __launch_bounds__(kTcRows) k_closure_infer_tc(closure_dev cd, co
       }
       const bool done = mbar_wait(bar, parity);
       parity ^= 1u;
-      ok = __syncthreads_and(done) != 0;
+      if (!done) s_fail[group] = 1;
+      group_sync(group);
+      ok = s_fail[group] == 0;
       if (!ok) break;
       tc_fence_after();
       if (layer < 3) {
@@ -936,7 +997,8 @@ __global__ void __launch_bounds__(kTcRows) k_closure_infer_tc(closure_dev cd, co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcTmemCols));
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr_s), "r"(kCols));
 }
 
 zsmpm_status cerr(zsmpm_status st, const std::string &m) { return (zsmpm_status)record_error(st, m.c_str()); }
@@ -1041,17 +1103,18 @@ bool closure_device_view(const zsmpm_closure *c, closure_dev *out) {
   return true;
 }
 
-// the G2P queue's network pass: the split-BF16 tcgen05 forward (three CTAs of 72 KB per SM)
+// the G2P queue's network pass: the split-BF16 tcgen05 forward
 cudaError_t launch_closure_rows(const closure_dev &cd, const float *x, float *y, const int *n_dev, long long cap,
                                 cudaStream_t st) {
-  k_closure_infer_tc<true><<<sms() * 3, kTcRows, kTcSplitSmem, st>>>(cd, cd.umma_w, x, y, cap, n_dev, cd.tc_status);
+  k_closure_infer_tc<true, kTcGroups><<<sms(), kTcRows * kTcGroups, kTcSplitSmem, st>>>(cd, cd.umma_w, x, y, cap, n_dev,
+                                                                                       cd.tc_status);
   return cudaGetLastError();
 }
 
 // the split variant's shared memory exceeds the 48 KB default: set once per device, before any
 // capture of its launches
 cudaError_t prepare_closure_kernels() {
-  return cudaFuncSetAttribute(k_closure_infer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSplitSmem);
+  return cudaFuncSetAttribute(k_closure_infer_tc<true, kTcGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSplitSmem);
 }
 }  // namespace zsmpm
 
@@ -1298,12 +1361,12 @@ ZSMPM_API zsmpm_status zsmpm_closure_infer(zsmpm_closure *c, const float *x, flo
       // six resident CTAs per SM (37.7 KB of shared memory and 64 tensor-memory columns each), so
       // that six tiles' layer chains overlap on the SM's tensor core
       const int grid = (int)std::min<int64_t>(tiles, (int64_t)sms() * 6);
-      k_closure_infer_tc<false><<<grid, kTcRows, kTcSmem, st>>>(c->cd, c->umma_w, x, y, n, nullptr, c->tc_status);
+      k_closure_infer_tc<false, 1><<<grid, kTcRows, kTcSmem, st>>>(c->cd, c->umma_w, x, y, n, nullptr, c->tc_status);
     } else {
       CZ_TRY(prepare_closure_kernels(), "closure kernel attributes");
-      const int grid = (int)std::min<int64_t>(tiles, (int64_t)sms() * 3);
-      k_closure_infer_tc<true><<<grid, kTcRows, kTcSplitSmem, st>>>(c->cd, c->umma_w, x, y, n, nullptr,
-                                                                    c->tc_status);
+      const int grid = (int)std::min<int64_t>(tiles, (int64_t)sms());
+      k_closure_infer_tc<true, kTcGroups><<<grid, kTcRows * kTcGroups, kTcSplitSmem, st>>>(c->cd, c->umma_w, x, y, n,
+                                                                                           nullptr, c->tc_status);
     }
   } else if (bf16) {
     const zsmpm_status ps = pack(c, st);
