@@ -872,13 +872,25 @@ __global__ void __launch_bounds__(kThreads) k_inc_finalize(scene_device s) {
 // The same passes as above in one cooperative kernel, with grid barriers in place of the kernel
 // boundaries: eight of them instead of 25 launches.  Scans over few entries (the bitmap's words,
 // the blocks) are done by every CTA for itself.  A launch boundary costs about 2.5 us here, a
-// barrier about 1 us, so this is the path wherever the passes are short (fused_prepare).
-constexpr int kPrepThreads = 512;
+// grid barrier about 2 us and a cluster barrier a fraction of one, so this is the path wherever the
+// passes are short (fused_prepare).
+//   kCluster: one cluster of 16 CTAs of 1,024 threads, synchronised by the hardware's cluster barrier;
+//   else a cooperative grid of 512-thread CTAs with a barrier in memory.
 constexpr int kPrepScan = 4096;  // entries a CTA scans by itself
+constexpr int kPrepCluster = 16;
+template <bool kCluster>
+struct prep_shape {
+  static constexpr int kThreads = kCluster ? 1024 : 512;
+};
 
 // All CTAs of the (cooperative) grid arrive; false when the wait gave up (kStatusTimeout is set and the
 // caller leaves).  `target` counts the arrivals up to and with this barrier.
+template <bool kCluster>
 __device__ __forceinline__ bool prep_barrier(const scene_device &s, int &target, int *ok) {
+  if (kCluster) {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    return true;
+  }
   target += gridDim.x;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -898,7 +910,7 @@ __device__ __forceinline__ bool prep_barrier(const scene_device &s, int &target,
 }
 
 // Exclusive scan of load(0 .. n) by this CTA into out[0 .. n] (shared memory, n <= kPrepScan)
-template <class Load>
+template <int kPrepThreads, class Load>
 __device__ __forceinline__ void prep_scan_local(Load load, int n, int *out, int *sm) {
   const int per = (n + kPrepThreads - 1) / kPrepThreads, lo = min(n, (int)threadIdx.x * per), hi = min(n, lo + per);
   int sum = 0;
@@ -913,16 +925,17 @@ __device__ __forceinline__ void prep_scan_local(Load load, int n, int *out, int 
 }
 
 // The same over many entries, with the whole grid, into out[0 .. n] in global memory (two barriers)
-template <class Load>
+template <bool kCluster, class Load>
 __device__ __forceinline__ bool prep_scan_grid(const scene_device &s, Load load, int n, int *out, int *sm, int &target,
                                                int *ok) {
+  constexpr int kPrepThreads = prep_shape<kCluster>::kThreads;
   const int chunk = (n + gridDim.x - 1) / gridDim.x;
   const int lo = min(n, (int)blockIdx.x * chunk), hi = min(n, lo + chunk);
   int acc = 0, total;
   for (int i = lo + threadIdx.x; i < hi; i += kPrepThreads) acc += load(i);
   cta_exclusive_scan<kPrepThreads>(acc, total, sm);
   if (threadIdx.x == 0) s.scan_part[blockIdx.x] = total;
-  if (!prep_barrier(s, target, ok)) return false;
+  if (!prep_barrier<kCluster>(s, target, ok)) return false;
   int before = 0, run;
   for (int i = threadIdx.x; i < (int)blockIdx.x; i += kPrepThreads) before += s.scan_part[i];
   cta_exclusive_scan<kPrepThreads>(before, run, sm);
@@ -933,7 +946,7 @@ __device__ __forceinline__ bool prep_scan_grid(const scene_device &s, Load load,
     run += total;
   }
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = run;
-  return prep_barrier(s, target, ok);
+  return prep_barrier<kCluster>(s, target, ok);
 }
 
 // cell starts, a warp per block (16 consecutive cells a lane), and the work order
@@ -975,7 +988,10 @@ __device__ __forceinline__ void prep_cell_start(const scene_device &s, int nb, c
   }
 }
 
-__global__ void __launch_bounds__(kPrepThreads, 2) k_prepare(scene_device s, int activate, int bin) {
+template <bool kCluster>
+__global__ void __launch_bounds__(prep_shape<kCluster>::kThreads, kCluster ? 1 : 2)
+    k_prepare(scene_device s, int activate, int bin) {
+  constexpr int kPrepThreads = prep_shape<kCluster>::kThreads;
   __shared__ int sm[kPrepThreads / 32 + 1];
   __shared__ int s_ok;
   __shared__ int s_scan[kPrepScan + 1];
@@ -984,25 +1000,25 @@ __global__ void __launch_bounds__(kPrepThreads, 2) k_prepare(scene_device s, int
   do {
     if (activate) {
       do_begin(s);
-      if (!prep_barrier(s, target, &s_ok)) break;
+      if (!prep_barrier<kCluster>(s, target, &s_ok)) break;
       do_insert_particle_blocks(s);
       do_insert_moved_blocks(s);
-      if (!prep_barrier(s, target, &s_ok)) break;
+      if (!prep_barrier<kCluster>(s, target, &s_ok)) break;
       do_enlarge(s);
-      if (!prep_barrier(s, target, &s_ok)) break;
+      if (!prep_barrier<kCluster>(s, target, &s_ok)) break;
       int nb, words;
       block_totals(s, blockIdx.x == 0 && threadIdx.x == 0, nb, words);
       do_bitmap_set(s, words > 0 ? nb : 0);
-      if (!prep_barrier(s, target, &s_ok)) break;
+      if (!prep_barrier<kCluster>(s, target, &s_ok)) break;
       const load_popc popc{s.bitmap};
       if (words <= kPrepScan) {
-        prep_scan_local(popc, words, s_scan, sm);
+        prep_scan_local<kPrepThreads>(popc, words, s_scan, sm);
         do_assign_ranks(s, words > 0 ? nb : 0, s_scan);
       } else {
-        if (!prep_scan_grid(s, popc, words, s.word_prefix, sm, target, &s_ok)) break;
+        if (!prep_scan_grid<kCluster>(s, popc, words, s.word_prefix, sm, target, &s_ok)) break;
         do_assign_ranks(s, nb, s.word_prefix);
       }
-      if (!prep_barrier(s, target, &s_ok)) break;
+      if (!prep_barrier<kCluster>(s, target, &s_ok)) break;
       do_neighbors(s);
     }
     if (bin) {
@@ -1010,19 +1026,19 @@ __global__ void __launch_bounds__(kPrepThreads, 2) k_prepare(scene_device s, int
       do_bin_count(s);
       do_inc_stayers<true>(s);
       do_inc_movers(s);
-      if (!prep_barrier(s, target, &s_ok)) break;
+      if (!prep_barrier<kCluster>(s, target, &s_ok)) break;
       const int nb = s.ctr[kCtrBlocks];
       const load_int count{s.block_count};
       if (nb < kPrepScan) {
-        prep_scan_local(count, nb, s_scan, sm);
+        prep_scan_local<kPrepThreads>(count, nb, s_scan, sm);
         if (blockIdx.x == 0)
           for (int i = threadIdx.x; i <= nb; i += kPrepThreads) s.block_start[i] = s_scan[i];
         prep_cell_start(s, nb, s_scan);
       } else {
-        if (!prep_scan_grid(s, count, nb, s.block_start, sm, target, &s_ok)) break;
+        if (!prep_scan_grid<kCluster>(s, count, nb, s.block_start, sm, target, &s_ok)) break;
         prep_cell_start(s, nb, s.block_start);
       }
-      if (!prep_barrier(s, target, &s_ok)) break;
+      if (!prep_barrier<kCluster>(s, target, &s_ok)) break;
       const bool inc = incremental_binning(s);
       do_bin_scatter(s);
       do_inc_place_stayers(s);
@@ -1031,7 +1047,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) k_prepare(scene_device s, int
       const long long quads = (long long)nb * (kGridChannels * 512 / 4);
       for (long long q = blockIdx.x * (long long)kPrepThreads + threadIdx.x; q < quads; q += grid_threads())
         reinterpret_cast<float4 *>(s.grid)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (!prep_barrier(s, target, &s_ok)) break;
+      if (!prep_barrier<kCluster>(s, target, &s_ok)) break;
       // the cells' lists by upload id (incremental: those that received movers), and the counts
       // zeroed for the next binning; a cell's length from the starts
       auto cell_len = [&](int j) {
@@ -1057,6 +1073,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) k_prepare(scene_device s, int
       }
     }
   } while (false);
+  if (kCluster) return;
   // the last CTA to leave clears the barrier for the next launch
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -2992,28 +3009,38 @@ int num_sms() {
 }  // namespace
 
 // ----------------------------------------------------------------- launchers
-// Whether activation and binning run as one cooperative launch (k_prepare): where the particles are few
+// Whether activation and binning run as one launch (k_prepare): where the particles are few
 // enough that the passes cost less than the launches' boundaries.
-// Measured, substep with and without it: 4 k particles 0.071 / 0.091 ms, 140 k 0.095 / 0.109, 490 k
-// 0.167 / 0.171, 3.7 M 0.515 / 0.510, 16 M 2.06 / 1.98.  With a learned closure the closure pass
-// runs beside activation and binning, and a cooperative grid waits for room beside it (3.7 M:
-// 1.09 / 1.03 ms), so those scenes keep the launches.
-constexpr int kPrepMaxParticles = 1 << 20;
+// Measured, substep with the launches / a cooperative grid / a cluster: 4 k particles 0.091 / 0.067 /
+// 0.062 ms, 140 k 0.109 / 0.096 / 0.102, 490 k 0.171 / 0.165 / 0.194, 3.7 M 0.510 / 0.515 / -, 16 M
+// 1.98 / 2.06 / -.  With a learned closure the closure pass runs beside activation and binning, and a
+// cooperative grid waits for room beside it (3.7 M: 1.03 / 1.09 ms), so those scenes keep the launches.
+constexpr int kPrepMaxParticles = 1 << 20, kPrepClusterParticles = 1 << 15;
 bool fused_prepare(const scene_device &s) { return s.prm.cap <= kPrepMaxParticles && !s.aux.learned; }
 
 cudaError_t launch_prepare(scene_device &s, bool activate, bool bin, cudaStream_t st) {
   const int sm = num_sms();
+  const bool cluster = s.prm.cap <= kPrepClusterParticles;
   cudaLaunchConfig_t cfg = {};
-  // about four particles a thread, at most two CTAs per SM (all CTAs are resident at once)
-  cfg.gridDim = dim3((unsigned)std::min(2 * sm, std::max(64, s.prm.n / (4 * kPrepThreads))));
-  cfg.blockDim = dim3(kPrepThreads);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_prepare, s, activate ? 1 : 0, bin ? 1 : 0);
+  if (cluster) {
+    cfg.gridDim = dim3(kPrepCluster);
+    cfg.blockDim = dim3(prep_shape<true>::kThreads);
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kPrepCluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    return cudaLaunchKernelEx(&cfg, k_prepare<true>, s, activate ? 1 : 0, bin ? 1 : 0);
+  }
+  // about four particles a thread, at most two CTAs per SM (all CTAs are resident at once)
+  constexpr int nt = prep_shape<false>::kThreads;
+  cfg.gridDim = dim3((unsigned)std::min(2 * sm, std::max(64, s.prm.n / (4 * nt))));
+  cfg.blockDim = dim3(nt);
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  return cudaLaunchKernelEx(&cfg, k_prepare<false>, s, activate ? 1 : 0, bin ? 1 : 0);
 }
 
 cudaError_t launch_activate(scene_device &s, cudaStream_t st) {
@@ -3068,6 +3095,8 @@ cudaError_t prepare_kernels() {
   p2g_attrs((const void *)k_p2g<true, 2>, 8);
   p2g_attrs((const void *)k_p2g<true, 3>, 12);
   p2g_attrs((const void *)k_p2g<true, 4>, 16);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_prepare<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_g2p2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG2P2GSmem);
   if (e != cudaSuccess) return e;
