@@ -1108,9 +1108,10 @@ __global__ void __launch_bounds__(prep_shape<kCluster>::kThreads, kCluster ? 1 :
 // (dx not a power of two) its weights are evaluated at f just outside [0.5, 1.5): the quadratic
 // B-spline is C1 there, so the difference is of second order in that rounding.
 //
-// What bounds it: instruction issue, about 300 thread instructions a particle (27 nodes x 4
-// channels x 2 operations in pairs, 108; weights, staging and emission the rest); the 68 bytes a
-// particle are 0.31 ms of a 30 M-particle launch.
+// What bounds it: the FMA pipe and instruction issue together, about 300 thread instructions a
+// particle (27 nodes x 4 channels x 2 operations in pairs, 108; weights, staging and emission the
+// rest); the 68 bytes a particle are 0.31 ms of a 30 M-particle launch.  That launch takes 0.947 ms
+// (0.996 with the weights in pairs too, 0.59 of it without the arithmetic of the nodes).
 constexpr int kP2GThreads = 128;
 constexpr int kP2GRanksDefault = 8;  // ranks in flight per cell unless tuned: windows of 4, 2 deep
 constexpr int kP2GWin = 4;            // ranks per window
@@ -1159,25 +1160,24 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 
 // Twice the quadratic B-spline weights (InterpolationKernel.hpp:93-130) of the nodes 0, 1, 2 of a
-// stencil for nh = 1 - f, the distance from the particle to the middle node in cells, in both
-// halves of a pair.  (The factor two drops the halvings; it is a power of two, so the products
-// of three such weights with data scaled by 1/8 round as the plain ones do.)
-__device__ __forceinline__ void bspline_weights2(float2 nh, float2 *w) {
-  const float2 t = add2(nh, dup2(0.5f));
-  w[0] = mul2(t, t);
-  w[1] = fma2(mul2(nh, dup2(-2.f)), nh, dup2(1.5f));
-  const float2 g = fma2(nh, dup2(-1.f), dup2(0.5f));
-  w[2] = mul2(g, g);
+// stencil for nh = 1 - f, the distance from the particle to the middle node in cells.  (The factor
+// two drops the halvings; it is a power of two, so the products of three such weights with data
+// scaled by 1/8 round as the plain ones do.)
+__device__ __forceinline__ void bspline_weights(float nh, float *w) {
+  const float t = nh + 0.5f, g = 0.5f - nh;
+  w[0] = t * t;
+  w[1] = fmaf(-2.f * nh, nh, 1.5f);
+  w[2] = g * g;
 }
 
 // Twice the node weights of the cell-centric pair (P2C2GTransfer): a particle's tent weights to
 // the centers of its two cells per axis, 1/2 - fx and 1/2 + fx with fx = x/dx - floor(x/dx + 1/2),
 // each passed half to either corner, over the nodes base .. base + 2 (base = floor(x/dx + 1/2)
 // - 1, fx = -nh).
-__device__ __forceinline__ void cell_weights2(float2 nh, float2 *w) {
-  w[0] = add2(nh, dup2(0.5f));
-  w[1] = dup2(1.f);
-  w[2] = fma2(nh, dup2(-1.f), dup2(0.5f));
+__device__ __forceinline__ void cell_weights(float nh, float *w) {
+  w[0] = nh + 0.5f;
+  w[1] = 1.f;
+  w[2] = 0.5f - nh;
 }
 
 // Parts a block's eight x planes are split into (work items of 8 / parts planes each): one where
@@ -1351,25 +1351,29 @@ __global__ void __launch_bounds__(kP2GThreads, 4) k_p2g(scene_device s, const fl
               } else {
                 X[0] = over_dx(prm, xm.x), X[1] = over_dx(prm, xm.y), X[2] = over_dx(prm, xm.z);
               }
-              const float2 hx = dup2(bx - X[0]), hy = dup2(by - X[1]), hz = dup2(bz - X[2]);
+              const float hx = bx - X[0], hy = by - X[1], hz = bz - X[2];
               // W (qm + (ii - 1) ax + (jj - 1) ay + (kk - 1) az): qm the momentum the middle node
               // would take, a the affine terms of one cell
               const float2 ax = mul2(make_float2(ra.y, rb.y), dx8), ay = mul2(make_float2(ra.z, rb.z), dx8),
                            az = mul2(make_float2(ra.w, rb.w), dx8);
               float2 q = mul2(dup2(xm.w * mscale), make_float2(ra.x, rb.x));
-              q = fma2(ax, hx, q);
-              q = fma2(ay, hy, q);
-              q = fma2(az, hz, q);
-              float2 wx[3], wy[3], wz[3];
+              q = fma2(ax, dup2(hx), q);
+              q = fma2(ay, dup2(hy), q);
+              q = fma2(az, dup2(hz), q);
+              // the weights are the channels' common factor: scalars, as a packed operation takes the
+              // FMA pipe 2.6 cycles a warp against 1.0 to 1.5 for a scalar one (measured), so packing
+              // pays by its issue slots where both halves differ and costs where they are the same
+              float wx[3], wy[3], w2[3];
               if (kCell) {
-                cell_weights2(hx, wx);
-                cell_weights2(hy, wy);
-                cell_weights2(hz, wz);
+                cell_weights(hx, wx);
+                cell_weights(hy, wy);
+                cell_weights(hz, w2);
               } else {
-                bspline_weights2(hx, wx);
-                bspline_weights2(hy, wy);
-                bspline_weights2(hz, wz);
+                bspline_weights(hx, wx);
+                bspline_weights(hy, wy);
+                bspline_weights(hz, w2);
               }
+              const float2 wz[3] = {dup2(w2[0]), dup2(w2[1]), dup2(w2[2])};
               const float2 minus = dup2(-1.f);
               const float2 c0 = mul2(mul2(wz[0], az), minus), c2 = mul2(wz[2], az);
 #pragma unroll
@@ -1378,7 +1382,7 @@ __global__ void __launch_bounds__(kP2GThreads, 4) k_p2g(scene_device s, const fl
 #pragma unroll
                 for (int jj = 0; jj < 3; ++jj) {
                   const float2 qij = jj == 0 ? fma2(ay, minus, qi) : jj == 1 ? qi : add2(qi, ay);
-                  const float2 wij = mul2(wx[ii], wy[jj]);
+                  const float2 wij = dup2(wx[ii] * wy[jj]);
                   const int n = (ii * 3 + jj) * 3;
                   acc[n] = fma2(wij, fma2(wz[0], qij, c0), acc[n]);
                   acc[n + 1] = fma2(wij, mul2(wz[1], qij), acc[n + 1]);
