@@ -1392,7 +1392,7 @@ ZSMPM_API zsmpm_status zsmpm_implicit_multiply(zsmpm_scene *s, const float *in, 
   cudaStream_t cs = as_stream(stream);
   ZS_TRY(cudaMemsetAsync(out, 0, sizeof(float) * (size_t)ndofs, cs), "multiply: zero");
   ZS_TRY(launch_g2p2g(s->dev, in, out, ndofs, dt, nullptr, cs), "multiply: g2p2g");
-  ZS_TRY(launch_implicit_mass(s->dev, in, out, dt, ndofs, nullptr, cs), "multiply: mass");
+  ZS_TRY(launch_implicit_mass(s->dev, in, out, dt, ndofs, cs), "multiply: mass");
   s->last_stream = cs;
   return ZSMPM_OK;
 }
@@ -1400,7 +1400,7 @@ ZSMPM_API zsmpm_status zsmpm_implicit_multiply(zsmpm_scene *s, const float *in, 
 ZSMPM_API zsmpm_status zsmpm_implicit_project(zsmpm_scene *s, float *inout, int64_t ndofs, void *stream) {
   zsmpm_status st = check_implicit(s, {inout}, ndofs);
   if (st != ZSMPM_OK) return st;
-  ZS_TRY(launch_implicit_project(s->dev, inout, ndofs, nullptr, as_stream(stream)), "project");
+  ZS_TRY(launch_implicit_project(s->dev, inout, ndofs, as_stream(stream)), "project");
   s->last_stream = as_stream(stream);
   return ZSMPM_OK;
 }
@@ -1409,7 +1409,7 @@ ZSMPM_API zsmpm_status zsmpm_implicit_precondition(zsmpm_scene *s, const float *
                                                    void *stream) {
   zsmpm_status st = check_implicit(s, {in, out}, ndofs);
   if (st != ZSMPM_OK) return st;
-  ZS_TRY(launch_implicit_precondition(s->dev, in, out, ndofs, nullptr, as_stream(stream)), "precondition");
+  ZS_TRY(launch_implicit_precondition(s->dev, in, out, ndofs, as_stream(stream)), "precondition");
   s->last_stream = as_stream(stream);
   return ZSMPM_OK;
 }
@@ -1435,15 +1435,18 @@ ZSMPM_API zsmpm_status zsmpm_implicit_cg(zsmpm_scene *s, float *x, const float *
       s->cg_buf = nullptr;
       s->cg_cap = 0;
     }
-    ZS_ALLOC(s->cg_buf, 4 * (size_t)stride, "cg scratch");
+    ZS_ALLOC(s->cg_buf, 3 * (size_t)stride, "cg scratch");
     s->cg_cap = stride;
   }
-  const cg_vectors v{s->cg_buf, s->cg_buf + stride, s->cg_buf + 2 * stride, s->cg_buf + 3 * stride};
-  ZS_TRY(launch_cg_begin(s->dev, x, b, v, ndofs, dt, s->cg, o.tol, o.rel_tol, cs), "cg begin");
+  const cg_vectors v{s->cg_buf, s->cg_buf + stride, s->cg_buf + 2 * stride};
+  ZS_TRY(launch_cg_begin(s->dev, x, b, v, ndofs, dt, s->cg, o.tol, o.rel_tol, o.max_iters, cs), "cg begin");
+  // eight iterations between the reads of the state: those that a finished solve skips cost four
+  // empty launches each, a read costs a round trip
   constexpr int kChunk = 8;
   cg_state h{};
-  for (int it = 0; it < o.max_iters + 1; it += kChunk) {
-    for (int k = 0; k < kChunk; ++k) ZS_TRY(launch_cg_iteration(s->dev, x, v, ndofs, dt, s->cg, o.max_iters, cs), "cg iteration");
+  for (int it = 0; it < o.max_iters; it += kChunk) {
+    for (int k = it; k < std::min(it + kChunk, o.max_iters); ++k)
+      ZS_TRY(launch_cg_iteration(s->dev, x, v, ndofs, dt, s->cg, o.max_iters, cs), "cg iteration");
     ZS_TRY(cudaMemcpyAsync(&h, s->cg, sizeof(cg_state), cudaMemcpyDeviceToHost, cs), "cg state");
     ZS_TRY(cudaStreamSynchronize(cs), "cg iteration");
     if (h.done) break;

@@ -205,28 +205,28 @@ int kernels_per_substep(const scene_device &s);
 // activation and binning in one launch (where fused_prepare says so)
 bool fused_prepare(const scene_device &s);
 cudaError_t launch_prepare(scene_device &s, bool activate, bool bin, cudaStream_t st);
-// the implicit system (ImplicitMPM.hpp) over node-major dof vectors [nb * 512 * 3]; a kernel
-// returns at once when `skip` (device, may be null) holds a nonzero value
+// the implicit system (ImplicitMPM.hpp) over node-major dof vectors [nb * 512 * 3]; the force
+// operator returns at once when `skip` (device, may be null) holds a nonzero value
 cudaError_t launch_g2p2g(scene_device &s, const float *v, float *f, long long ndofs, float dt, const int *skip,
                          cudaStream_t st);
 cudaError_t launch_implicit_mass(scene_device &s, const float *dv, float *out, float dt, long long ndofs,
-                                 const int *skip, cudaStream_t st);
-cudaError_t launch_implicit_project(scene_device &s, float *dof, long long ndofs, const int *skip,
-                                    cudaStream_t st);
+                                 cudaStream_t st);
+cudaError_t launch_implicit_project(scene_device &s, float *dof, long long ndofs, cudaStream_t st);
 cudaError_t launch_implicit_precondition(scene_device &s, const float *in, float *out, long long ndofs,
-                                         const int *skip, cudaStream_t st);
+                                         cudaStream_t st);
 
 // ConjugateGradient::solve state on the device
 struct cg_state {
   double acc;        // dot product accumulator (zeroed by its consumer)
   float ztrk, norm, local_tol, alpha, beta;
   int done, iter;
+  unsigned arrived;  // CTAs that have added to acc
 };
 struct cg_vectors {
-  float *r, *p, *q, *ap;  // residual, search direction, preconditioned residual, A p
+  float *r, *p, *ap;  // residual, search direction, A p
 };
-cudaError_t launch_cg_begin(scene_device &s, float *x, const float *b, const cg_vectors &v, long long ndofs, float dt,
-                            cg_state *cs, float tol, float rel_tol, cudaStream_t st);
+cudaError_t launch_cg_begin(scene_device &s, const float *x, const float *b, const cg_vectors &v, long long ndofs,
+                            float dt, cg_state *cs, float tol, float rel_tol, int max_iters, cudaStream_t st);
 cudaError_t launch_cg_iteration(scene_device &s, float *x, const cg_vectors &v, long long ndofs, float dt,
                                 cg_state *cs, int max_iters, cudaStream_t st);
 

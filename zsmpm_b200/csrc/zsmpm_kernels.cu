@@ -2511,12 +2511,33 @@ __device__ __forceinline__ long long dof_count(const scene_device &s, long long 
   return 0;
 }
 
+// mass of the node t = block * 512 + cell
+__device__ __forceinline__ float node_mass(const scene_device &s, long long t) {
+  return s.grid[(t >> 9) * kGridChannels * 512 + (t & 511)];
+}
+// the collision response of the scene's walls, colliders and level sets at a node
+struct node_boundaries {
+  const scene_params &p;
+  int ncol, nls;
+  __device__ __forceinline__ explicit node_boundaries(const scene_params &prm)
+      : p(prm),
+        ncol(prm.ncolliders ? min(*prm.ncolliders, kMaxColliders) : 0),
+        nls(prm.nlevelsets ? min(*prm.nlevelsets, kMaxLevelsets) : 0) {}
+  __device__ __forceinline__ void apply(const scene_device &s, long long t, float v[3]) const {
+    const int cell = (int)(t & 511);
+    const int3 k = unpack_key(s.blk_pk[t >> 9]);
+    const float pos[3] = {((float)k.x * 8.f + (float)(cell >> 6)) * p.dx,
+                          ((float)k.y * 8.f + (float)((cell >> 3) & 7)) * p.dx,
+                          ((float)k.z * 8.f + (float)(cell & 7)) * p.dx};
+    apply_walls(p, pos, v);
+    if (ncol + nls > 0) apply_colliders(p, ncol, nls, pos, v);
+  }
+};
+
 // ImplicitMPMSystem::ForceDtSqrPlusMass (ImplicitMPM.hpp:17-33): where the grid mass of the
 // node is positive, out = (f dt^2 + m) dv, with f = out on entry.
 __global__ void __launch_bounds__(kThreads) k_implicit_mass(scene_device s, const float *__restrict__ dv,
-                                                             float *__restrict__ out, float dt, long long ndofs,
-                                                             const int *skip) {
-  if (skip && *skip) return;
+                                                             float *__restrict__ out, float dt, long long ndofs) {
   const long long total = dof_count(s, ndofs);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += grid_threads()) {
     const long long node = i / 3;
@@ -2528,23 +2549,14 @@ __global__ void __launch_bounds__(kThreads) k_implicit_mass(scene_device s, cons
 // ImplicitMPMSystem::Projector (ImplicitMPM.hpp:63-97) with the scene's six walls: nodes with
 // positive mass get the walls' collision response, all others are zeroed.
 __global__ void __launch_bounds__(kThreads) k_implicit_project(scene_device s, float *__restrict__ dof,
-                                                                long long ndofs, const int *skip) {
-  if (skip && *skip) return;
-  const scene_params &p = s.prm;
+                                                                long long ndofs) {
+  const node_boundaries bc(s.prm);
   const long long total = dof_count(s, ndofs) / 3;
-  const int ncol = p.ncolliders ? min(*p.ncolliders, kMaxColliders) : 0;
-  const int nls = p.nlevelsets ? min(*p.nlevelsets, kMaxLevelsets) : 0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += grid_threads()) {
-    const int b = (int)(t >> 9), cell = (int)(t & 511);
     float *v = dof + t * 3;
-    if (s.grid[(size_t)b * kGridChannels * 512 + cell] > 0.f) {
-      const int3 k = unpack_key(s.blk_pk[b]);
-      const float pos[3] = {((float)k.x * 8.f + (float)(cell >> 6)) * p.dx,
-                            ((float)k.y * 8.f + (float)((cell >> 3) & 7)) * p.dx,
-                            ((float)k.z * 8.f + (float)(cell & 7)) * p.dx};
+    if (node_mass(s, t) > 0.f) {
       float vel[3] = {v[0], v[1], v[2]};
-      apply_walls(p, pos, vel);
-      if (ncol + nls > 0) apply_colliders(p, ncol, nls, pos, vel);
+      bc.apply(s, t, vel);
       v[0] = vel[0];
       v[1] = vel[1];
       v[2] = vel[2];
@@ -2557,9 +2569,7 @@ __global__ void __launch_bounds__(kThreads) k_implicit_project(scene_device s, f
 // ImplicitMPMSystem::DivPernodeMass (ImplicitMPM.hpp:126-137): out = in / m where the grid
 // mass is positive; other entries of out are left as they are.
 __global__ void __launch_bounds__(kThreads) k_implicit_precondition(scene_device s, const float *__restrict__ in,
-                                                                     float *__restrict__ out, long long ndofs,
-                                                                     const int *skip) {
-  if (skip && *skip) return;
+                                                                     float *__restrict__ out, long long ndofs) {
   const long long total = dof_count(s, ndofs);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += grid_threads()) {
     const long long node = i / 3;
@@ -2570,104 +2580,164 @@ __global__ void __launch_bounds__(kThreads) k_implicit_precondition(scene_device
 
 // ConjugateGradient::solve (math/linear/ConjugateGradient.hpp:69-172) on the device.  The
 // scalars (r.q, alpha, beta, the stopping test) live in a cg_state in device memory, so no
-// step needs the host: every kernel of an iteration returns at once when the iteration's
-// check found the solve finished.  Dot products sum float products per thread and warp, and
-// the warp sums in double.
+// step needs the host: every kernel of an iteration returns at once when the solve is finished.
+//
+// An iteration is four launches: the force operator, and three passes over the nodes that do
+// between two dot products all that needs no other node (mass, boundaries and p.Ap; the updates of
+// x and r, the preconditioner and r.q; the new direction and a zeroed A p).  The CTA that arrives
+// last at a dot product takes its scalars.  The vectors stay in L2 (7 MB each for 3.7 M particles),
+// so a pass costs mostly its launch and the reduction: ten iterations and the start, force operator
+// included, take 5.11 ms where launches of one operation each took 5.97 (50 k: 1.03 and 1.56).
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
   return v;
 }
 
-__global__ void __launch_bounds__(kThreads) k_cg_fill0(scene_device s, float *__restrict__ v, long long ndofs,
-                                                        const int *skip) {
-  if (skip && *skip) return;
-  const long long total = dof_count(s, ndofs);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += grid_threads()) v[i] = 0.f;
-}
-
-// r = b - Ax (ConjugateGradient.hpp:97-98)
-__global__ void __launch_bounds__(kThreads) k_cg_residual(scene_device s, const float *__restrict__ b,
-                                                           const float *__restrict__ ax, float *__restrict__ r,
-                                                           long long ndofs) {
-  const long long total = dof_count(s, ndofs);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += grid_threads())
-    r[i] = b[i] - ax[i];
-}
-
-__global__ void __launch_bounds__(kThreads) k_cg_copy(scene_device s, const float *__restrict__ src,
-                                                       float *__restrict__ dst, long long ndofs) {
-  const long long total = dof_count(s, ndofs);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += grid_threads()) dst[i] = src[i];
-}
-
-__global__ void __launch_bounds__(kThreads) k_cg_dot(scene_device s, const float *__restrict__ a,
-                                                      const float *__restrict__ b, long long ndofs, cg_state *cs) {
-  if (cs->done) return;
-  const long long total = dof_count(s, ndofs);
-  float acc = 0.f;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += grid_threads())
-    acc += a[i] * b[i];
+// Adds the CTA's products (floats per thread and warp, doubles from there on) to the dot product;
+// true in thread 0 of the CTA that arrives last, with the sum in out and the accumulator cleared.
+__device__ __forceinline__ bool cg_dot(float acc, cg_state *cs, double &out) {
+  __shared__ double s_sum[kThreads / 32];
   acc = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0 && acc != 0.f) atomicAdd(&cs->acc, (double)acc);
-}
-
-// after the first r.q: the norm and the tolerance min(relTol * norm, tol) (:115-117)
-__global__ void k_cg_init(cg_state *cs, float tol, float rel_tol) {
-  const float z = (float)cs->acc;
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = (double)acc;
+  __syncthreads();
+  if (threadIdx.x != 0) return false;
+  double sum = 0.0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) sum += s_sum[w];
+  if (sum != 0.0) atomicAdd(&cs->acc, sum);
+  __threadfence();
+  if (atomicAdd(&cs->arrived, 1u) != gridDim.x - 1) return false;
+  __threadfence();
+  out = atomicAdd(&cs->acc, 0.0);
   cs->acc = 0.0;
-  cs->ztrk = z;
-  cs->norm = sqrtf(z);
-  cs->local_tol = fminf(rel_tol * cs->norm, tol);
-  cs->iter = 0;
-  cs->done = 0;
+  cs->arrived = 0;
+  return true;
 }
 
 // the loop head (:118-122): stop at the tolerance or after max_iters iterations
-__global__ void k_cg_check(cg_state *cs, int max_iters) {
-  if (cs->done) return;
+__device__ __forceinline__ void cg_check(cg_state *cs, int max_iters) {
   if (cs->iter >= max_iters || cs->norm <= cs->local_tol) cs->done = 1;
 }
 
-__global__ void k_cg_alpha(cg_state *cs) {
-  if (cs->done) return;
-  cs->alpha = cs->ztrk / (float)cs->acc;  // alpha = zTrk / (Ap . p)  (:134)
-  cs->acc = 0.0;
+// ForceDtSqrPlusMass and Projector on one node: v = the constrained (f dt^2 + m) d, zero off the mass
+__device__ __forceinline__ void cg_operator(const scene_device &s, const node_boundaries &bc, long long t, float m,
+                                            const float *f, const float *d, float dt, float v[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v[k] = (f[3 * t + k] * dt * dt + m) * d[3 * t + k];
+  bc.apply(s, t, v);
 }
 
-// x = alpha p + x, r = -alpha Ap + r (:137-143)
-__global__ void __launch_bounds__(kThreads) k_cg_update_xr(scene_device s, float *__restrict__ x, float *__restrict__ r,
-                                                            const float *__restrict__ p, const float *__restrict__ ap,
-                                                            long long ndofs, const cg_state *cs) {
-  if (cs->done) return;
-  const float alpha = cs->alpha;
-  const long long total = dof_count(s, ndofs);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += grid_threads()) {
-    x[i] = alpha * p[i] + x[i];
-    r[i] = -alpha * ap[i] + r[i];
+// The solve's start from A x's forces in ap: r = P(b - A x), p = M r, zTrk = r.p, and the tolerance
+// min(relTol * norm, tol) (:97-117); A p zeroed for the first iteration's forces.
+__global__ void __launch_bounds__(kThreads) k_cg_start(scene_device s, const float *__restrict__ x,
+                                                        const float *__restrict__ b, cg_vectors v, long long ndofs,
+                                                        float dt, cg_state *cs, float tol, float rel_tol,
+                                                        int max_iters) {
+  const node_boundaries bc(s.prm);
+  const long long total = dof_count(s, ndofs) / 3;
+  float acc = 0.f;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += grid_threads()) {
+    const float m = node_mass(s, t);
+    float r[3] = {0.f, 0.f, 0.f}, q[3] = {0.f, 0.f, 0.f};
+    if (m > 0.f) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const float ax = (v.ap[3 * t + k] * dt * dt + m) * x[3 * t + k];
+        r[k] = b[3 * t + k] - ax;
+      }
+      bc.apply(s, t, r);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) q[k] = r[k] / m;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      v.r[3 * t + k] = r[k];
+      v.p[3 * t + k] = q[k];
+      v.ap[3 * t + k] = 0.f;
+      acc += r[k] * q[k];
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.ctr[kCtrWork + kWorkG2P2G] = 0;
+  double dot;
+  if (cg_dot(acc, cs, dot)) {
+    const float z = (float)dot;
+    cs->ztrk = z;
+    cs->norm = sqrtf(z);
+    cs->local_tol = fminf(rel_tol * cs->norm, tol);
+    cg_check(cs, max_iters);
   }
 }
 
-// zTrk = q.r, beta = zTrk / zTrkLast, norm = sqrt(zTrk), one iteration done (:156-170)
-__global__ void k_cg_beta(cg_state *cs) {
+// A p from its forces, and alpha = zTrk / (Ap . p) (:129-134)
+__global__ void __launch_bounds__(kThreads) k_cg_apply(scene_device s, cg_vectors v, long long ndofs, float dt,
+                                                        cg_state *cs) {
   if (cs->done) return;
-  const float last = cs->ztrk;
-  cs->ztrk = (float)cs->acc;
-  cs->acc = 0.0;
-  cs->beta = cs->ztrk / last;
-  cs->norm = sqrtf(cs->ztrk);
-  cs->iter += 1;
+  const node_boundaries bc(s.prm);
+  const long long total = dof_count(s, ndofs) / 3;
+  float acc = 0.f;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += grid_threads()) {
+    const float m = node_mass(s, t);
+    if (!(m > 0.f)) continue;  // p, r and A p are zero there
+    float a[3];
+    cg_operator(s, bc, t, m, v.ap, v.p, dt, a);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      v.ap[3 * t + k] = a[k];
+      acc += a[k] * v.p[3 * t + k];
+    }
+  }
+  double dot;
+  if (cg_dot(acc, cs, dot)) cs->alpha = cs->ztrk / (float)dot;
 }
 
-// p = beta p + q (:163)
-__global__ void __launch_bounds__(kThreads) k_cg_update_p(scene_device s, float *__restrict__ p,
-                                                           const float *__restrict__ q, long long ndofs,
-                                                           const cg_state *cs) {
+// x = alpha p + x, r = -alpha Ap + r, zTrk = r . M r, beta = zTrk / zTrkLast, norm = sqrt(zTrk),
+// one iteration done (:137-170)
+__global__ void __launch_bounds__(kThreads) k_cg_update(scene_device s, float *__restrict__ x, cg_vectors v,
+                                                         long long ndofs, cg_state *cs, int max_iters) {
+  if (cs->done) return;
+  const float alpha = cs->alpha;
+  const long long total = dof_count(s, ndofs) / 3;
+  float acc = 0.f;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += grid_threads()) {
+    const float m = node_mass(s, t);
+    if (!(m > 0.f)) continue;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const long long i = 3 * t + k;
+      x[i] = alpha * v.p[i] + x[i];
+      const float r = -alpha * v.ap[i] + v.r[i];
+      v.r[i] = r;
+      acc += r / m * r;
+    }
+  }
+  double dot;
+  if (cg_dot(acc, cs, dot)) {
+    const float last = cs->ztrk;
+    cs->ztrk = (float)dot;
+    cs->beta = cs->ztrk / last;
+    cs->norm = sqrtf(cs->ztrk);
+    cs->iter += 1;
+    cg_check(cs, max_iters);
+  }
+}
+
+// p = beta p + M r (:163), and the next iteration's A p zeroed
+__global__ void __launch_bounds__(kThreads) k_cg_direction(scene_device s, cg_vectors v, long long ndofs,
+                                                            const cg_state *cs) {
   if (cs->done) return;
   const float beta = cs->beta;
-  const long long total = dof_count(s, ndofs);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += grid_threads())
-    p[i] = beta * p[i] + q[i];
+  const long long total = dof_count(s, ndofs) / 3;
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.ctr[kCtrWork + kWorkG2P2G] = 0;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += grid_threads()) {
+    const float m = node_mass(s, t);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const long long i = 3 * t + k;
+      if (m > 0.f) v.p[i] = beta * v.p[i] + v.r[i] / m;
+      v.ap[i] = 0.f;
+    }
+  }
 }
 
 // ----------------------------------------------------------------- import / export
@@ -3219,60 +3289,47 @@ cudaError_t launch_g2p2g(scene_device &s, const float *v, float *f, long long nd
 }
 
 cudaError_t launch_implicit_mass(scene_device &s, const float *dv, float *out, float dt, long long ndofs,
-                                 const int *skip, cudaStream_t st) {
-  k_implicit_mass<<<num_sms() * 4, kThreads, 0, st>>>(s, dv, out, dt, ndofs, skip);
+                                 cudaStream_t st) {
+  k_implicit_mass<<<num_sms() * 4, kThreads, 0, st>>>(s, dv, out, dt, ndofs);
   return cudaGetLastError();
 }
 
-cudaError_t launch_implicit_project(scene_device &s, float *dof, long long ndofs, const int *skip,
-                                    cudaStream_t st) {
-  k_implicit_project<<<num_sms() * 4, kThreads, 0, st>>>(s, dof, ndofs, skip);
+cudaError_t launch_implicit_project(scene_device &s, float *dof, long long ndofs, cudaStream_t st) {
+  k_implicit_project<<<num_sms() * 4, kThreads, 0, st>>>(s, dof, ndofs);
   return cudaGetLastError();
 }
 
 cudaError_t launch_implicit_precondition(scene_device &s, const float *in, float *out, long long ndofs,
-                                         const int *skip, cudaStream_t st) {
-  k_implicit_precondition<<<num_sms() * 4, kThreads, 0, st>>>(s, in, out, ndofs, skip);
+                                         cudaStream_t st) {
+  k_implicit_precondition<<<num_sms() * 4, kThreads, 0, st>>>(s, in, out, ndofs);
   return cudaGetLastError();
 }
 
-// The solve's start: r = b - A x, project r, q = M r (q zeroed first), p = q, zTrk = r.q.
-cudaError_t launch_cg_begin(scene_device &s, float *x, const float *b, const cg_vectors &v, long long ndofs, float dt,
-                            cg_state *cs, float tol, float rel_tol, cudaStream_t st) {
-  const int grid = num_sms() * 4;
+// CTAs of a pass over the nodes that ndofs admits (at most four per SM)
+static int cg_grid(long long ndofs) {
+  return (int)std::max(1ll, std::min(4ll * num_sms(), (ndofs / 3 + kThreads - 1) / kThreads));
+}
+
+// The solve's start: r = b - A x, project r, p = M r, zTrk = r.p, and the loop's first check.
+cudaError_t launch_cg_begin(scene_device &s, const float *x, const float *b, const cg_vectors &v, long long ndofs,
+                            float dt, cg_state *cs, float tol, float rel_tol, int max_iters, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(cs, 0, sizeof(cg_state), st);
   if (e != cudaSuccess) return e;
-  k_cg_fill0<<<grid, kThreads, 0, st>>>(s, v.ap, ndofs, nullptr);
+  if ((e = cudaMemsetAsync(v.ap, 0, sizeof(float) * (size_t)ndofs, st)) != cudaSuccess) return e;
   if ((e = launch_g2p2g(s, x, v.ap, ndofs, dt, nullptr, st)) != cudaSuccess) return e;
-  if ((e = launch_implicit_mass(s, x, v.ap, dt, ndofs, nullptr, st)) != cudaSuccess) return e;
-  k_cg_residual<<<grid, kThreads, 0, st>>>(s, b, v.ap, v.r, ndofs);
-  if ((e = launch_implicit_project(s, v.r, ndofs, nullptr, st)) != cudaSuccess) return e;
-  k_cg_fill0<<<grid, kThreads, 0, st>>>(s, v.q, ndofs, nullptr);
-  if ((e = launch_implicit_precondition(s, v.r, v.q, ndofs, nullptr, st)) != cudaSuccess) return e;
-  k_cg_copy<<<grid, kThreads, 0, st>>>(s, v.q, v.p, ndofs);
-  k_cg_dot<<<grid, kThreads, 0, st>>>(s, v.r, v.q, ndofs, cs);
-  k_cg_init<<<1, 1, 0, st>>>(cs, tol, rel_tol);
+  k_cg_start<<<cg_grid(ndofs), kThreads, 0, st>>>(s, x, b, v, ndofs, dt, cs, tol, rel_tol, max_iters);
   return cudaGetLastError();
 }
 
 // One loop iteration (ConjugateGradient.hpp:118-171); does nothing once the solve is done.
 cudaError_t launch_cg_iteration(scene_device &s, float *x, const cg_vectors &v, long long ndofs, float dt,
                                 cg_state *cs, int max_iters, cudaStream_t st) {
-  const int grid = num_sms() * 4;
-  const int *done = &cs->done;
-  k_cg_check<<<1, 1, 0, st>>>(cs, max_iters);
-  k_cg_fill0<<<grid, kThreads, 0, st>>>(s, v.ap, ndofs, done);
-  cudaError_t e = launch_g2p2g(s, v.p, v.ap, ndofs, dt, done, st);
-  if (e != cudaSuccess) return e;
-  if ((e = launch_implicit_mass(s, v.p, v.ap, dt, ndofs, done, st)) != cudaSuccess) return e;
-  if ((e = launch_implicit_project(s, v.ap, ndofs, done, st)) != cudaSuccess) return e;
-  k_cg_dot<<<grid, kThreads, 0, st>>>(s, v.ap, v.p, ndofs, cs);
-  k_cg_alpha<<<1, 1, 0, st>>>(cs);
-  k_cg_update_xr<<<grid, kThreads, 0, st>>>(s, x, v.r, v.p, v.ap, ndofs, cs);
-  if ((e = launch_implicit_precondition(s, v.r, v.q, ndofs, done, st)) != cudaSuccess) return e;
-  k_cg_dot<<<grid, kThreads, 0, st>>>(s, v.q, v.r, ndofs, cs);
-  k_cg_beta<<<1, 1, 0, st>>>(cs);
-  k_cg_update_p<<<grid, kThreads, 0, st>>>(s, v.p, v.q, ndofs, cs);
+  const int grid = cg_grid(ndofs);
+  // its work counter was cleared by the pass before
+  k_g2p2g<<<num_sms() * 2, kG2P2GThreads, kG2P2GSmem, st>>>(s, v.p, v.ap, ndofs, dt, &cs->done);
+  k_cg_apply<<<grid, kThreads, 0, st>>>(s, v, ndofs, dt, cs);
+  k_cg_update<<<grid, kThreads, 0, st>>>(s, x, v, ndofs, cs, max_iters);
+  k_cg_direction<<<grid, kThreads, 0, st>>>(s, v, ndofs, cs);
   return cudaGetLastError();
 }
 
