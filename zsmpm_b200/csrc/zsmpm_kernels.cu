@@ -1110,8 +1110,8 @@ __global__ void __launch_bounds__(prep_shape<kCluster>::kThreads, kCluster ? 1 :
 //
 // What bounds it: the FMA pipe and instruction issue together, about 300 thread instructions a
 // particle (27 nodes x 4 channels x 2 operations in pairs, 108; weights, staging and emission the
-// rest); the 68 bytes a particle are 0.31 ms of a 30 M-particle launch.  That launch takes 0.947 ms
-// (0.996 with the weights in pairs too, 0.59 of it without the arithmetic of the nodes).
+// rest); the 68 bytes a particle are 0.31 ms of a 30 M-particle launch.  That launch takes 0.918 ms
+// (0.59 of it without the arithmetic of the nodes, 0.17 for the flush).
 constexpr int kP2GThreads = 128;
 constexpr int kP2GRanksDefault = 8;  // ranks in flight per cell unless tuned: windows of 4, 2 deep
 constexpr int kP2GWin = 4;            // ranks per window
@@ -1158,6 +1158,10 @@ __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+// acc + w v as two scalar operations
+__device__ __forceinline__ float2 add_scaled(float2 acc, float w, float2 v) {
+  return make_float2(fmaf(w, v.x, acc.x), fmaf(w, v.y, acc.y));
+}
 
 // Twice the quadratic B-spline weights (InterpolationKernel.hpp:93-130) of the nodes 0, 1, 2 of a
 // stencil for nh = 1 - f, the distance from the particle to the middle node in cells.  (The factor
@@ -1360,9 +1364,11 @@ __global__ void __launch_bounds__(kP2GThreads, 4) k_p2g(scene_device s, const fl
               q = fma2(ax, dup2(hx), q);
               q = fma2(ay, dup2(hy), q);
               q = fma2(az, dup2(hz), q);
-              // the weights are the channels' common factor: scalars, as a packed operation takes the
-              // FMA pipe 2.6 cycles a warp against 1.0 to 1.5 for a scalar one (measured), so packing
-              // pays by its issue slots where both halves differ and costs where they are the same
+              // A packed operation takes the FMA pipe 2.6 cycles a warp, a scalar one 1.0 to 1.5
+              // (measured): packing saves issue slots and costs pipe time.  The balance: the weights, the
+              // channels' common factor, and the sums as scalars, the nodes' values in pairs (30 M
+              // particles: all in pairs 0.996 ms, scalar weights 0.947, scalar sums too 0.918, all scalar
+              // 0.928).
               float wx[3], wy[3], w2[3];
               if (kCell) {
                 cell_weights(hx, wx);
@@ -1382,11 +1388,11 @@ __global__ void __launch_bounds__(kP2GThreads, 4) k_p2g(scene_device s, const fl
 #pragma unroll
                 for (int jj = 0; jj < 3; ++jj) {
                   const float2 qij = jj == 0 ? fma2(ay, minus, qi) : jj == 1 ? qi : add2(qi, ay);
-                  const float2 wij = dup2(wx[ii] * wy[jj]);
+                  const float wij = wx[ii] * wy[jj];
                   const int n = (ii * 3 + jj) * 3;
-                  acc[n] = fma2(wij, fma2(wz[0], qij, c0), acc[n]);
-                  acc[n + 1] = fma2(wij, mul2(wz[1], qij), acc[n + 1]);
-                  acc[n + 2] = fma2(wij, fma2(wz[2], qij, c2), acc[n + 2]);
+                  acc[n] = add_scaled(acc[n], wij, fma2(wz[0], qij, c0));
+                  acc[n + 1] = add_scaled(acc[n + 1], wij, mul2(wz[1], qij));
+                  acc[n + 2] = add_scaled(acc[n + 2], wij, fma2(wz[2], qij, c2));
                 }
               }
               xm = xm_n, ra = ra_n, rb = rb_n;
