@@ -1378,7 +1378,7 @@ ZSMPM_API zsmpm_status zsmpm_g2p2g(zsmpm_scene *s, const float *v, float *f, int
   zsmpm_status st = check_implicit(s, {v, f}, ndofs);
   if (st != ZSMPM_OK) return st;
   if (!std::isfinite(dt)) return fail(ZSMPM_ERR_INVALID_ARG, "dt must be finite");
-  ZS_TRY(launch_g2p2g(s->dev, v, f, ndofs, dt, nullptr, as_stream(stream)), "g2p2g");
+  ZS_TRY(launch_g2p2g(s->dev, v, f, ndofs, dt, as_stream(stream)), "g2p2g");
   s->last_stream = as_stream(stream);
   return ZSMPM_OK;
 }
@@ -1391,7 +1391,7 @@ ZSMPM_API zsmpm_status zsmpm_implicit_multiply(zsmpm_scene *s, const float *in, 
   if (in == out) return fail(ZSMPM_ERR_INVALID_ARG, "multiply needs distinct in and out vectors");
   cudaStream_t cs = as_stream(stream);
   ZS_TRY(cudaMemsetAsync(out, 0, sizeof(float) * (size_t)ndofs, cs), "multiply: zero");
-  ZS_TRY(launch_g2p2g(s->dev, in, out, ndofs, dt, nullptr, cs), "multiply: g2p2g");
+  ZS_TRY(launch_g2p2g(s->dev, in, out, ndofs, dt, cs), "multiply: g2p2g");
   ZS_TRY(launch_implicit_mass(s->dev, in, out, dt, ndofs, cs), "multiply: mass");
   s->last_stream = cs;
   return ZSMPM_OK;

@@ -78,8 +78,8 @@ enum work_slot : int {
   kWorkFinalize = 1,
   kWorkP2G = 2,
   kWorkG2P = 3,
-  kWorkGrid = 4,
-  kWorkG2P2G = 5  // reset by its own launcher (the operator runs many times per activation)
+  kWorkForceRows = 4,  // reset by their launcher (the operator runs many times per activation)
+  kWorkForceScatter = 5
 };
 
 struct scene_params {
@@ -205,10 +205,8 @@ int kernels_per_substep(const scene_device &s);
 // activation and binning in one launch (where fused_prepare says so)
 bool fused_prepare(const scene_device &s);
 cudaError_t launch_prepare(scene_device &s, bool activate, bool bin, cudaStream_t st);
-// the implicit system (ImplicitMPM.hpp) over node-major dof vectors [nb * 512 * 3]; the force
-// operator returns at once when `skip` (device, may be null) holds a nonzero value
-cudaError_t launch_g2p2g(scene_device &s, const float *v, float *f, long long ndofs, float dt, const int *skip,
-                         cudaStream_t st);
+// the implicit system (ImplicitMPM.hpp) over node-major dof vectors [nb * 512 * 3]
+cudaError_t launch_g2p2g(scene_device &s, const float *v, float *f, long long ndofs, float dt, cudaStream_t st);
 cudaError_t launch_implicit_mass(scene_device &s, const float *dv, float *out, float dt, long long ndofs,
                                  cudaStream_t st);
 cudaError_t launch_implicit_project(scene_device &s, float *dof, long long ndofs, cudaStream_t st);

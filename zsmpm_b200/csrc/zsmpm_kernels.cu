@@ -1194,9 +1194,11 @@ __device__ __forceinline__ int plane_parts(int nb, int ctas) {
 // kCell: P2C2GTransfer of the cell-centric pair (below) with the pair's node weights and affine
 // term; `rows` holds v and the affine term (A = m C - (4 dt/dx^2) tau for APIC), with_mass = 0
 // leaves the mass channel and the m v term out.  S windows in the ring (the staging depth of the
-// tuner: 8, 12 or 16 ranks).
-template <bool kCell, int S>
-__global__ void __launch_bounds__(kP2GThreads, 4) k_p2g(scene_device s, const float4 *rows, int with_mass) {
+// tuner: 8, 12 or 16 ranks).  kDof: the second half of G2P2G (below), which adds the three vector
+// channels to the node-major dof vector fout (ndofs entries).
+template <bool kCell, int S, bool kDof = false>
+__global__ void __launch_bounds__(kP2GThreads, 4)
+    k_p2g(scene_device s, const float4 *rows, int with_mass, float *fout, long long ndofs, const int *skip) {
   extern __shared__ __align__(16) float4 p2g_smem[];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   float4 *const ring = p2g_smem + w * S * kP2GStage;
@@ -1209,8 +1211,9 @@ __global__ void __launch_bounds__(kP2GThreads, 4) k_p2g(scene_device s, const fl
   __shared__ unsigned char s_hot[4][4];  // [node plane][warp]: the warp added to it
   const scene_params &prm = s.prm;
   const int nb = s.ctr[kCtrBlocks], front = s.ctr[kCtrOrderFront], nwork = work_blocks(s);
+  if (kDof && ((skip && *skip) || (long long)nb * 1536 > ndofs)) return;  // (k_force_rows sets the status)
   const int parts = plane_parts(nwork, gridDim.x), nx = 8 / parts, items = nwork * parts;
-  int *const counter = &s.ctr[kCtrWork + kWorkP2G];
+  int *const counter = &s.ctr[kCtrWork + (kDof ? kWorkForceScatter : kWorkP2G)];
   for (int q = t; q < kP2GUnit; q += kP2GThreads) unit[q] = make_float4(1.f, 0.f, 0.f, 0.f);
   for (int q = t; q < 16 * kP2GPlane; q += kP2GThreads) plane[q] = 0.f;
 
@@ -1441,27 +1444,47 @@ __global__ void __launch_bounds__(kP2GThreads, 4) k_p2g(scene_device s, const fl
       // ---- flush the two planes: each 4 channels x 10 y x 3 quads of z, a row summed over the two
       // warps that share it, by 16-byte reductions into the blocks b + {0,1}^3; the next two planes
       // go to the other buffers, so one barrier is enough
-      for (int it = t; it < 120 * min(2, nx + 2 - p0); it += kP2GThreads) {
-        const int p = it < 120 ? 0 : 1, u = it - 120 * p;
-        const int ch = u / 30, hy = u % 30 / 3, quad = u % 3;
-        const float *const at = pl0 + p * 4 * kP2GPlane + ch * kP2GPlaneCh + quad * 4;
-        const int v = hy >> 1, row = hy & 1;
-        float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (v < 4 && s_hot[(p0 & 2) + p][v])
-          q4 = *reinterpret_cast<const float4 *>(at + v * kP2GPlane + row * kP2GPlaneRow);
-        if (v > 0 && s_hot[(p0 & 2) + p][v - 1]) {
-          const float4 o = *reinterpret_cast<const float4 *>(at + (v - 1) * kP2GPlane + (row + 2) * kP2GPlaneRow);
-          q4.x += o.x, q4.y += o.y, q4.z += o.z, q4.w += o.w;
-        }
-        if (q4.x != 0.f || q4.y != 0.f || q4.z != 0.f || q4.w != 0.f) {
-          const int X = x0 + p0 + p + 1, Y = hy + 1;
-          const int tb = cs[kMetaNbr + ((X >= 8 ? 4 : 0) | (Y >= 8 ? 2 : 0) | (quad == 2 ? 1 : 0))];
-          if (tb < 0)
-            set_status(s.ctr, kStatusMissingBlock);
-          else
-            red_add_v4(s.grid + ((size_t)tb * kGridChannels + ch) * 512 +
-                           (((X & 7) << 6) | ((Y & 7) << 3) | ((quad * 4) & 7)),
-                       q4.x, q4.y, q4.z, q4.w);
+      // (kDof: 10 y x 3 quads, the three vector channels of a quad's nodes as three of them)
+      constexpr int kItems = kDof ? 30 : 120;
+      for (int it = t; it < kItems * min(2, nx + 2 - p0); it += kP2GThreads) {
+        const int p = it < kItems ? 0 : 1, u = it - kItems * p;
+        const int hy = u % 30 / 3, quad = u % 3, v = hy >> 1, row = hy & 1;
+        const bool lo = v < 4 && s_hot[(p0 & 2) + p][v], hi = v > 0 && s_hot[(p0 & 2) + p][v - 1];
+        auto quad_sum = [&](int ch) {
+          const float *const at = pl0 + p * 4 * kP2GPlane + ch * kP2GPlaneCh + quad * 4;
+          float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (lo) q4 = *reinterpret_cast<const float4 *>(at + v * kP2GPlane + row * kP2GPlaneRow);
+          if (hi) {
+            const float4 o = *reinterpret_cast<const float4 *>(at + (v - 1) * kP2GPlane + (row + 2) * kP2GPlaneRow);
+            q4.x += o.x, q4.y += o.y, q4.z += o.z, q4.w += o.w;
+          }
+          return q4;
+        };
+        auto nonzero = [](float4 q) { return q.x != 0.f || q.y != 0.f || q.z != 0.f || q.w != 0.f; };
+        const int X = x0 + p0 + p + 1, Y = hy + 1;
+        const int cell = ((X & 7) << 6) | ((Y & 7) << 3) | ((quad * 4) & 7);
+        const int *const to = cs + kMetaNbr + ((X >= 8 ? 4 : 0) | (Y >= 8 ? 2 : 0) | (quad == 2 ? 1 : 0));
+        if (kDof) {
+          const float4 fx = quad_sum(1), fy = quad_sum(2), fz = quad_sum(3);
+          if (nonzero(fx) || nonzero(fy) || nonzero(fz)) {
+            if (*to < 0) {
+              set_status(s.ctr, kStatusMissingBlock);
+            } else {
+              float *const dst = fout + ((size_t)*to * 512 + cell) * 3;
+              red_add_v4(dst, fx.x, fy.x, fz.x, fx.y);
+              red_add_v4(dst + 4, fy.y, fz.y, fx.z, fy.z);
+              red_add_v4(dst + 8, fz.z, fx.w, fy.w, fz.w);
+            }
+          }
+        } else {
+          const int ch = u / 30;
+          const float4 q4 = quad_sum(ch);
+          if (nonzero(q4)) {
+            if (*to < 0)
+              set_status(s.ctr, kStatusMissingBlock);
+            else
+              red_add_v4(s.grid + ((size_t)*to * kGridChannels + ch) * 512 + cell, q4.x, q4.y, q4.z, q4.w);
+          }
         }
       }
     }
@@ -2215,41 +2238,27 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 5) k_g2p(scene_device s) {
 
 // ----------------------------------------------------------------- G2P2G and the implicit system
 // G2P2GTransfer (simulation/transfer/G2P2G.hpp:49-142), the force operator of the implicit
-// solve (simulation/mpm/ImplicitMPM.hpp:34-61).  One CTA per block (persistent); the velocity
-// field is staged in a 12^3 halo of float4 nodes.  The block's 512 cells are processed in
-// chunks of 64, in two phases as in P2G:
-//  1. consecutive threads take consecutive particles of the chunk: gather C, form the trial
-//     F = (I + dt C) F, evaluate the stress on a copy of the state (nothing is written back),
-//     and stage the particle's weights and its force in the affine form
-//     f(node) = W (q + ii a_x + jj a_y + kk a_z), (a_x a_y a_z) = (4/dx) tau, q = -(4/dx) tau f,
-//     which equals W (4/dx^2) tau (x_i - x_p) with node offsets (ii, jj, kk) in cells;
-//  2. one thread per (cell, component) sums the staged particles of its cell into 27
-//     registers (all particles of a cell share the 27 nodes) and adds them to a 12^3 force
-//     halo in shared memory, which is flushed into f with 16-byte reductions.
-// Against one shared atomic per particle, node and component (81 per particle, limited by the
-// shared-atomic rate) the staging takes the kernel from 3.6 to 2.95 ms on 30 M particles.
+// solve (simulation/mpm/ImplicitMPM.hpp:34-61), in two launches:
+//  1. k_force_rows: per particle, gather C from the velocity vector, form the trial
+//     F = (I + dt C) F, evaluate the stress on a copy of the state (the particle's own is not
+//     written) and store (4/dx^2) tau as the particle's affine rows (in the next buffer, which the
+//     next G2P overwrites);
+//  2. k_p2g<kDof> scatters them, f(node) += W (4/dx^2) tau (x_i - x_p), as P2G does the affine
+//     momentum, into the force vector.
 // v and f are node-major over the active blocks in canonical order, v[(block*512 + cell)*3 + d]:
 // the layout of a dof_view<space, 3> over a Vector (types/View.h:77-168).
-constexpr int kG2P2GThreads = 256;
-constexpr int kG2P2GChunk = 64;
-constexpr int kG2P2GRanks = 11;   // particles per cell staged per chunk (more scatter directly)
-constexpr int kG2P2GFields = 21;  // w[9], q[3], ax[3], ay[3], az[3]
-constexpr int kG2P2GRow = kG2P2GChunk + 1;
-constexpr int kG2P2GMap = 1024;   // slots of a chunk mapped to their cell (more: binary search)
-constexpr size_t kG2P2GSmem = sizeof(float4) * kHaloCells + sizeof(float) * 3 * kHaloCells +
-                              sizeof(float) * kG2P2GFields * kG2P2GRanks * kG2P2GRow +
-                              sizeof(int) * 2 * (kG2P2GChunk + 1) + 2 * kG2P2GMap;
-
-__global__ void __launch_bounds__(kG2P2GThreads, 2)
-    k_g2p2g(scene_device s, const float *__restrict__ vin, float *__restrict__ fout, long long ndofs, float dt,
-            const int *skip) {
+//
+// One kernel that gathered a chunk of 64 cells, staged its particles in shared memory and added
+// their sums to a halo of forces there kept its two halves waiting for each other at 16 barriers a
+// block, and used one CTA a block however few there were; the rows cost 96 bytes a particle and
+// free both halves of that (ten iterations of the solve: 3.7 M particles 5.12 -> 4.02 ms, 50 k 1.04 ->
+// 0.56).  What bounds k_force_rows is instruction issue, as in k_g2p: the gather and the SVD.
+__global__ void __launch_bounds__(kThreads, 3)
+    k_force_rows(scene_device s, const float *__restrict__ vin, long long ndofs, float dt, const int *skip,
+                 float4 *rows) {
   if (skip && *skip) return;
-  extern __shared__ __align__(16) float gg_smem[];
-  float4 *svf = reinterpret_cast<float4 *>(gg_smem);
-  float *sf = gg_smem + 4 * kHaloCells;  // [3][kHaloCells]
-  auto stg = reinterpret_cast<float(*)[kG2P2GRanks][kG2P2GRow]>(sf + 3 * kHaloCells);
-  int *const s_cs0 = reinterpret_cast<int *>(sf + 3 * kHaloCells + kG2P2GFields * kG2P2GRanks * kG2P2GRow);
-  unsigned char *const s_map0 = reinterpret_cast<unsigned char *>(s_cs0 + 2 * (kG2P2GChunk + 1));
+  extern __shared__ __align__(16) float force_smem[];
+  float4 *const svf = reinterpret_cast<float4 *>(force_smem);
   __shared__ int s_b;
   const scene_params &p = s.prm;
   const int nb = s.ctr[kCtrBlocks], front = s.ctr[kCtrOrderFront], nwork = work_blocks(s);
@@ -2257,18 +2266,29 @@ __global__ void __launch_bounds__(kG2P2GThreads, 2)
     if (blockIdx.x == 0 && threadIdx.x == 0) set_status(s.ctr, kStatusCapacity);
     return;
   }
-  const int t = threadIdx.x;
-  const int my_cell = t % kG2P2GChunk, my_ch = t / kG2P2GChunk;
-  // the force halo starts zeroed; each block's flush zeroes the quads it sends (as in k_p2g)
-  for (int q = t; q < 3 * kHaloCells; q += kG2P2GThreads) sf[q] = 0.f;
+  const int parts = slot_parts(nwork, gridDim.x);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float scale = p.four_over_dx * p.inv_dx;
+  float *const pf = force_smem + 4 * kHaloCells + warp * 2 * kG2PPrefetch;
+  auto prefetch = [&](int buf, int i) {
+    float *b = pf + buf * kG2PPrefetch;
+    cp_async16(b + 4 * lane, &s.cur.xm[i]);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) cp_async4(b + 128 + 32 * k + lane, &s.cur.F[mat_at(k, i)]);
+    if (s.cur.plastic) cp_async4(b + 416 + lane, &s.cur.plastic[i]);
+    cp_async_commit();
+  };
   for (;;) {
-    const int w = grab_block(&s.ctr[kCtrWork + kWorkG2P2G], &s_b);
-    if (w >= nwork) break;
-    const int b = work_block(s, front, nb, w);
-    const int end = s.block_start[b + 1];
+    const int w = grab_block(&s.ctr[kCtrWork + kWorkForceRows], &s_b);
+    if (w >= nwork * parts) break;
+    const int b = work_block(s, front, nb, w / parts);
+    const int first = s.block_start[b], last = s.block_start[b + 1];
+    const int len = (last - first + 32 * parts - 1) / (32 * parts) * 32;
+    const int start = first + w % parts * len, end = min(last, start + len);
+    if (start >= end) continue;
     // velocity halo: items (hx, hy, quad) over 12 x 12 x 3; four consecutive nodes are 12
     // consecutive floats (three 16-byte loads)
-    for (int it = t; it < kHalo * kHalo * 3; it += kG2P2GThreads) {
+    for (int it = threadIdx.x; it < kHalo * kHalo * 3; it += kThreads) {
       const int quad = it % 3, hy = (it / 3) % kHalo, hx = it / (3 * kHalo);
       const int tb = s.nbr[b * 8 + ((hx >= 8 ? 4 : 0) | (hy >= 8 ? 2 : 0) | (quad == 2 ? 1 : 0))];
       float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a, d = a;
@@ -2285,225 +2305,98 @@ __global__ void __launch_bounds__(kG2P2GThreads, 2)
       dst[2] = make_float4(c.z, c.w, d.x, 0.f);
       dst[3] = make_float4(d.y, d.z, d.w, 0.f);
     }
+    __syncthreads();
     const int3 bk = unpack_key(s.blk_pk[b]);
     const int org[3] = {bk.x * 8, bk.y * 8, bk.z * 8};
-    // cell starts of chunk k in s_cs0 + (k & 1) * (kG2P2GChunk + 1) and its slot -> cell map in
-    // s_map0 + (k & 1) * kG2P2GMap; the next chunk's are filled during this chunk's phase 2
-    auto fill = [&](int k) {
-      if (t <= kG2P2GChunk) {
-        const int nc = k * kG2P2GChunk + t;
-        s_cs0[(k & 1) * (kG2P2GChunk + 1) + t] = nc < 512 ? s.cell_start[b * 512 + nc] : end;
-      }
-      if (t < kG2P2GChunk) {
-        const int c = k * kG2P2GChunk + t;
-        const int cs = s.cell_start[b * 512 + c];
-        const int ce = c + 1 < 512 ? s.cell_start[b * 512 + c + 1] : end;
-        const int base = s.cell_start[b * 512 + k * kG2P2GChunk];
-        unsigned char *m = s_map0 + (k & 1) * kG2P2GMap;
-        for (int q = cs - base; q < ce - base && q < kG2P2GMap; ++q) m[q] = (unsigned char)t;
-      }
-    };
-    fill(0);
-    for (int chunk = 0; chunk < 512 / kG2P2GChunk; ++chunk) {
-      const int cell0 = chunk * kG2P2GChunk;
-      __syncthreads();  // halos ready, previous staging consumed, this chunk's starts and map in place
-      const int *s_cs = s_cs0 + (chunk & 1) * (kG2P2GChunk + 1);
-      const unsigned char *s_map = s_map0 + (chunk & 1) * kG2P2GMap;
-      const int c0 = s_cs[0], c1 = s_cs[kG2P2GChunk];
-      // ---- phase 1 (the whole CTA steps together: the SVD's early exit is a warp vote, so
-      // lanes past the chunk's end run on a copy of its first particle and stage nothing)
-      for (int base = c0; base < c1; base += kG2P2GThreads) {
-        const int slot = base + t;
-        const bool active = slot < c1;
-        const int i = s.src[active ? slot : c0];
-        const float4 xm = s.cur.xm[i];
-        float F[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) F[k] = s.cur.F[mat_at(k, i)];
-        float pl = s.cur.plastic ? s.cur.plastic[i] : 0.f;
-        const float X[3] = {over_dx(p, xm.x), over_dx(p, xm.y), over_dx(p, xm.z)};
-        int hb[3];
-        float w[3][3], f[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const float bs = floorf(X[d] - 0.5f);
-          f[d] = X[d] - bs;
-          hb[d] = (int)bs - org[d];
-          w[d][0] = 0.5f * (1.5f - f[d]) * (1.5f - f[d]);
-          const float f1 = f[d] - 1.f;
-          w[d][1] = 0.75f - f1 * f1;
-          const float f2 = 0.5f + f1;
-          w[d][2] = 0.5f * f2 * f2;
-        }
-        const bool inside = hb[0] >= 0 && hb[0] <= kHalo - 3 && hb[1] >= 0 && hb[1] <= kHalo - 3 &&
-                            hb[2] >= 0 && hb[2] <= kHalo - 3;
-        if (active && !inside) set_status(s.ctr, kStatusMissingBlock);
-        float B[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // sum W v (node - f)^T
-        if (inside) {
-#pragma unroll
-          for (int ii = 0; ii < 3; ++ii) {
-            const float dxi = (float)ii - f[0];
-#pragma unroll
-            for (int jj = 0; jj < 3; ++jj) {
-              const float dyj = (float)jj - f[1];
-              const float wij = w[0][ii] * w[1][jj];
-              const int hrow = ((hb[0] + ii) * kHalo + (hb[1] + jj)) * kHalo + hb[2];
-              float s0[3] = {0.f, 0.f, 0.f}, s1[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-              for (int kk = 0; kk < 3; ++kk) {
-                const float wz = w[2][kk], wzd = wz * ((float)kk - f[2]);
-                const float4 node = svf[hrow + kk];
-                s0[0] += wz * node.x;
-                s0[1] += wz * node.y;
-                s0[2] += wz * node.z;
-                s1[0] += wzd * node.x;
-                s1[1] += wzd * node.y;
-                s1[2] += wzd * node.z;
-              }
-#pragma unroll
-              for (int d = 0; d < 3; ++d) {
-                const float a = wij * s0[d];
-                B[d] += a * dxi;
-                B[3 + d] += a * dyj;
-                B[6 + d] += wij * s1[d];
-              }
-            }
-          }
-        }
-        // trial F = (I + dt C) F (G2P2G.hpp:103-105), C = B 4/dx
-        float Fn[9];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int r = 0; r < 3; ++r)
-            Fn[3 * c + r] = F[3 * c + r] + dt * p.four_over_dx *
-                                               (B[r] * F[3 * c] + B[3 + r] * F[3 * c + 1] + B[6 + r] * F[3 * c + 2]);
-        float tau[9];
-        constitutive_update<true, false>(p.mat, Fn, pl, tau);
-        if (!active) continue;
-        float ax[3], ay[3], az[3], q[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          ax[d] = tau[d] * p.four_over_dx;
-          ay[d] = tau[3 + d] * p.four_over_dx;
-          az[d] = tau[6 + d] * p.four_over_dx;
-          q[d] = -(ax[d] * f[0] + ay[d] * f[1] + az[d] * f[2]);
-        }
-        int lo = 0;  // the cell of this slot: the last cell whose start is <= slot
-        if (slot - c0 < kG2P2GMap) {
-          lo = s_map[slot - c0];
-        } else {
-          int hi = kG2P2GChunk;
-          while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (s_cs[mid] <= slot) lo = mid;
-            else hi = mid;
-          }
-        }
-        const int cl = lo, r = slot - s_cs[lo], cell = cell0 + cl;
-        const bool on_cell = hb[0] == (cell >> 6) + 1 && hb[1] == ((cell >> 3) & 7) + 1 && hb[2] == (cell & 7) + 1;
-        if (r >= kG2P2GRanks || !on_cell) {
-          // beyond the staged ranks, or a stencil origin that rounding moved off the cell:
-          // scatter directly and stage a zero stand-in
-          if (inside)
-            for (int ii = 0; ii < 3; ++ii)
-              for (int jj = 0; jj < 3; ++jj)
-                for (int kk = 0; kk < 3; ++kk) {
-                  const float W = w[0][ii] * w[1][jj] * w[2][kk];
-                  const int h = ((hb[0] + ii) * kHalo + (hb[1] + jj)) * kHalo + hb[2] + kk;
-#pragma unroll
-                  for (int d = 0; d < 3; ++d)
-                    atomicAdd(&sf[d * kHaloCells + h],
-                              W * (q[d] + (float)ii * ax[d] + (float)jj * ay[d] + (float)kk * az[d]));
-                }
-          if (r < kG2P2GRanks)
-            for (int fl = 0; fl < kG2P2GFields; ++fl) stg[fl][r][cl] = 0.f;
-          continue;
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) stg[3 * a + c][r][cl] = w[a][c];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          stg[9 + d][r][cl] = q[d];
-          stg[12 + d][r][cl] = ax[d];
-          stg[15 + d][r][cl] = ay[d];
-          stg[18 + d][r][cl] = az[d];
-        }
-      }
-      __syncthreads();
-      if (chunk + 1 < 512 / kG2P2GChunk) fill(chunk + 1);
-      // ---- phase 2: thread (cell, component) sums the staged particles of its cell
-      const int cnt = my_ch < 3 ? min(s_cs[my_cell + 1] - s_cs[my_cell], kG2P2GRanks) : 0;
-      if (cnt > 0) {
-        const int d = my_ch;
-        float acc[27];
-#pragma unroll
-        for (int n = 0; n < 27; ++n) acc[n] = 0.f;
-        for (int r = 0; r < cnt; ++r) {
-          float w[3][3];
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) w[a][c] = stg[3 * a + c][r][my_cell];
-          const float q = stg[9 + d][r][my_cell];
-          const float ax = stg[12 + d][r][my_cell];
-          const float ay = stg[15 + d][r][my_cell];
-          const float az = stg[18 + d][r][my_cell];
-          const float cz1 = w[2][1] * az, cz2 = 2.f * w[2][2] * az;  // as in k_p2g
-#pragma unroll
-          for (int ii = 0; ii < 3; ++ii) {
-            const float qi = q + (float)ii * ax;
-#pragma unroll
-            for (int jj = 0; jj < 3; ++jj) {
-              const float qij = qi + (float)jj * ay;
-              const float wij = w[0][ii] * w[1][jj];
-              const int n = (ii * 3 + jj) * 3;
-              acc[n] = fmaf(wij, w[2][0] * qij, acc[n]);
-              acc[n + 1] = fmaf(wij, fmaf(w[2][1], qij, cz1), acc[n + 1]);
-              acc[n + 2] = fmaf(wij, fmaf(w[2][2], qij, cz2), acc[n + 2]);
-            }
-          }
-        }
-        const int cell = cell0 + my_cell;
-        const int ex = (cell >> 6) + 1, ey = ((cell >> 3) & 7) + 1, ez = (cell & 7) + 1;
-        float *dst = sf + d * kHaloCells;
-#pragma unroll
-        for (int ii = 0; ii < 3; ++ii)
-#pragma unroll
-          for (int jj = 0; jj < 3; ++jj)
-#pragma unroll
-            for (int kk = 0; kk < 3; ++kk)
-              atomicAdd(&dst[((ex + ii) * kHalo + (ey + jj)) * kHalo + ez + kk], acc[(ii * 3 + jj) * 3 + kk]);
-      }
+    // batches of 32 slots a warp, the next batch's particles copied meanwhile (as in k_g2p); lanes
+    // past the end work on a copy of the part's first particle, as the SVD's early exit is a warp vote
+    int buf = 0, i = 0, inext = 0;
+    const int base0 = start + warp * 32;
+    if (base0 < end) {
+      i = s.src[base0 + lane < end ? base0 + lane : start];
+      prefetch(0, i);
+      if (base0 + kThreads < end) inext = s.src[base0 + kThreads + lane < end ? base0 + kThreads + lane : start];
     }
-    __syncthreads();
-    // flush: items (hx, hy, quad); four nodes x three components = three 16-byte reductions
-    for (int it = t; it < kHalo * kHalo * 3; it += kG2P2GThreads) {
-      const int quad = it % 3, hy = (it / 3) % kHalo, hx = it / (3 * kHalo);
-      const int h = (hx * kHalo + hy) * kHalo + quad * 4;
-      float v[12];
+    for (int base = base0; base < end; base += kThreads) {
+      const bool active = base + lane < end;
+      const int nslot2 = base + 2 * kThreads + lane;
+      const int inext2 = base + 2 * kThreads < end ? s.src[nslot2 < end ? nslot2 : start] : 0;
+      cp_async_wait_all();
+      const float *const pb = pf + buf * kG2PPrefetch;
+      const float4 xm = reinterpret_cast<const float4 *>(pb)[lane];
+      const int icur = i;
+      if (base + kThreads < end) prefetch(buf ^ 1, inext);
+      buf ^= 1;
+      i = inext;
+      inext = inext2;
+      const float X[3] = {over_dx(p, xm.x), over_dx(p, xm.y), over_dx(p, xm.z)};
+      int hb[3];
+      float wt[3][3], f[3];
 #pragma unroll
-      for (int n = 0; n < 4; ++n)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) v[3 * n + d] = sf[d * kHaloCells + h + n];
-      bool any = false;
-#pragma unroll
-      for (int k = 0; k < 12; ++k) any = any || v[k] != 0.f;
-      if (!any) continue;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) *reinterpret_cast<float4 *>(&sf[d * kHaloCells + h]) = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int tb = s.nbr[b * 8 + ((hx >= 8 ? 4 : 0) | (hy >= 8 ? 2 : 0) | (quad == 2 ? 1 : 0))];
-      if (tb < 0) {
-        set_status(s.ctr, kStatusMissingBlock);
-        continue;
+      for (int d = 0; d < 3; ++d) {
+        const float bs = floorf(X[d] - 0.5f);
+        f[d] = X[d] - bs;
+        hb[d] = (int)bs - org[d];
+        wt[d][0] = 0.5f * (1.5f - f[d]) * (1.5f - f[d]);
+        const float f1 = f[d] - 1.f;
+        wt[d][1] = 0.75f - f1 * f1;
+        const float f2 = 0.5f + f1;
+        wt[d][2] = 0.5f * f2 * f2;
       }
-      const int cell = ((hx & 7) << 6) | ((hy & 7) << 3) | ((quad * 4) & 7);
-      float *dst = fout + ((size_t)tb * 512 + cell) * 3;
-      red_add_v4(dst, v[0], v[1], v[2], v[3]);
-      red_add_v4(dst + 4, v[4], v[5], v[6], v[7]);
-      red_add_v4(dst + 8, v[8], v[9], v[10], v[11]);
+      const bool inside = hb[0] >= 0 && hb[0] <= kHalo - 3 && hb[1] >= 0 && hb[1] <= kHalo - 3 && hb[2] >= 0 &&
+                          hb[2] <= kHalo - 3;
+      if (active && !inside) set_status(s.ctr, kStatusMissingBlock);
+      float B[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // sum W v (node - f)^T
+      if (inside) {
+#pragma unroll
+        for (int ii = 0; ii < 3; ++ii) {
+          const float dxi = (float)ii - f[0];
+#pragma unroll
+          for (int jj = 0; jj < 3; ++jj) {
+            const float dyj = (float)jj - f[1];
+            const float wij = wt[0][ii] * wt[1][jj];
+            const int hrow = ((hb[0] + ii) * kHalo + (hb[1] + jj)) * kHalo + hb[2];
+            float s0[3] = {0.f, 0.f, 0.f}, s1[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+            for (int kk = 0; kk < 3; ++kk) {
+              const float wz = wt[2][kk], wzd = wz * ((float)kk - f[2]);
+              const float4 node = svf[hrow + kk];
+              s0[0] += wz * node.x;
+              s0[1] += wz * node.y;
+              s0[2] += wz * node.z;
+              s1[0] += wzd * node.x;
+              s1[1] += wzd * node.y;
+              s1[2] += wzd * node.z;
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              const float a = wij * s0[d];
+              B[d] += a * dxi;
+              B[3 + d] += a * dyj;
+              B[6 + d] += wij * s1[d];
+            }
+          }
+        }
+      }
+      // trial F = (I + dt C) F (G2P2G.hpp:103-105), C = B 4/dx
+      float F[9], Fn[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) F[k] = pb[128 + 32 * k + lane];
+      float pl = s.cur.plastic ? pb[416 + lane] : 0.f;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+          Fn[3 * c + r] = F[3 * c + r] + dt * p.four_over_dx *
+                                             (B[r] * F[3 * c] + B[3 + r] * F[3 * c + 1] + B[6 + r] * F[3 * c + 2]);
+      float tau[9];
+      constitutive_update<true, false>(p.mat, Fn, pl, tau);
+      if (!active) continue;
+      // (a particle outside the halo scatters nothing)
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        rows[row_at(d, icur)] = inside ? make_float4(0.f, scale * tau[d], scale * tau[3 + d], scale * tau[6 + d])
+                                       : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
 }
@@ -2593,7 +2486,7 @@ __global__ void __launch_bounds__(kThreads) k_implicit_precondition(scene_device
 // x and r, the preconditioner and r.q; the new direction and a zeroed A p).  The CTA that arrives
 // last at a dot product takes its scalars.  The vectors stay in L2 (7 MB each for 3.7 M particles),
 // so a pass costs mostly its launch and the reduction: ten iterations and the start, force operator
-// included, take 5.11 ms where launches of one operation each took 5.97 (50 k: 1.03 and 1.56).
+// included, take 5.11 ms where launches of one operation each took 5.97 (50 k: 1.03 and 1.56; with the fused force operator of the time).
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
@@ -2664,7 +2557,7 @@ __global__ void __launch_bounds__(kThreads) k_cg_start(scene_device s, const flo
       acc += r[k] * q[k];
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) s.ctr[kCtrWork + kWorkG2P2G] = 0;
+  if (blockIdx.x == 0 && threadIdx.x < 2) s.ctr[kCtrWork + kWorkForceRows + threadIdx.x] = 0;
   double dot;
   if (cg_dot(acc, cs, dot)) {
     const float z = (float)dot;
@@ -2734,7 +2627,7 @@ __global__ void __launch_bounds__(kThreads) k_cg_direction(scene_device s, cg_ve
   if (cs->done) return;
   const float beta = cs->beta;
   const long long total = dof_count(s, ndofs) / 3;
-  if (blockIdx.x == 0 && threadIdx.x == 0) s.ctr[kCtrWork + kWorkG2P2G] = 0;
+  if (blockIdx.x == 0 && threadIdx.x < 2) s.ctr[kCtrWork + kWorkForceRows + threadIdx.x] = 0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += grid_threads()) {
     const float m = node_mass(s, t);
 #pragma unroll
@@ -3172,13 +3065,14 @@ cudaError_t prepare_kernels() {
   p2g_attrs((const void *)k_p2g<false, 2>, 8);
   p2g_attrs((const void *)k_p2g<false, 3>, 12);
   p2g_attrs((const void *)k_p2g<false, 4>, 16);
+  p2g_attrs((const void *)k_p2g<false, 2, true>, 8);
   p2g_attrs((const void *)k_p2g<true, 2>, 8);
   p2g_attrs((const void *)k_p2g<true, 3>, 12);
   p2g_attrs((const void *)k_p2g<true, 4>, 16);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_prepare<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_g2p2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG2P2GSmem);
+  e = cudaFuncSetAttribute(k_force_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2p_smem_bytes(kThreads));
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_g2p<true, true, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)g2p_smem_bytes(kThreads));
@@ -3212,11 +3106,11 @@ static void launch_staged_p2g(scene_device &s, const float4 *rows, int with_mass
   const int dflt = ranks == 8 ? 4 : ranks == 16 ? 2 : 3;
   const int grid = num_sms() * (s.prm.p2g_ctas_per_sm > 0 ? s.prm.p2g_ctas_per_sm : dflt);
   if (ranks == 8)
-    k_p2g<kCell, 2><<<grid, kP2GThreads, p2g_smem_bytes(8), st>>>(s, rows, with_mass);
+    k_p2g<kCell, 2><<<grid, kP2GThreads, p2g_smem_bytes(8), st>>>(s, rows, with_mass, nullptr, 0, nullptr);
   else if (ranks == 16)
-    k_p2g<kCell, 4><<<grid, kP2GThreads, p2g_smem_bytes(16), st>>>(s, rows, with_mass);
+    k_p2g<kCell, 4><<<grid, kP2GThreads, p2g_smem_bytes(16), st>>>(s, rows, with_mass, nullptr, 0, nullptr);
   else
-    k_p2g<kCell, 3><<<grid, kP2GThreads, p2g_smem_bytes(12), st>>>(s, rows, with_mass);
+    k_p2g<kCell, 3><<<grid, kP2GThreads, p2g_smem_bytes(12), st>>>(s, rows, with_mass, nullptr, 0, nullptr);
 }
 
 cudaError_t launch_p2g(scene_device &s, cudaStream_t st) {
@@ -3286,12 +3180,17 @@ cudaError_t launch_g2p(scene_device &s, cudaStream_t st, bool closure_pass) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_g2p2g(scene_device &s, const float *v, float *f, long long ndofs, float dt, const int *skip,
-                         cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(&s.ctr[kCtrWork + kWorkG2P2G], 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
-  k_g2p2g<<<num_sms() * 2, kG2P2GThreads, kG2P2GSmem, st>>>(s, v, f, ndofs, dt, skip);
+// the force operator's two kernels; both work counters are zero on entry
+static cudaError_t launch_force(scene_device &s, const float *v, float *f, long long ndofs, float dt, const int *skip,
+                                cudaStream_t st) {
+  k_force_rows<<<num_sms() * 3, kThreads, g2p_smem_bytes(kThreads), st>>>(s, v, ndofs, dt, skip, s.nxt.row);
+  k_p2g<false, 2, true><<<num_sms() * 4, kP2GThreads, p2g_smem_bytes(8), st>>>(s, s.nxt.row, 0, f, ndofs, skip);
   return cudaGetLastError();
+}
+
+cudaError_t launch_g2p2g(scene_device &s, const float *v, float *f, long long ndofs, float dt, cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(&s.ctr[kCtrWork + kWorkForceRows], 0, 2 * sizeof(int), st);
+  return e != cudaSuccess ? e : launch_force(s, v, f, ndofs, dt, nullptr, st);
 }
 
 cudaError_t launch_implicit_mass(scene_device &s, const float *dv, float *out, float dt, long long ndofs,
@@ -3322,7 +3221,7 @@ cudaError_t launch_cg_begin(scene_device &s, const float *x, const float *b, con
   cudaError_t e = cudaMemsetAsync(cs, 0, sizeof(cg_state), st);
   if (e != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(v.ap, 0, sizeof(float) * (size_t)ndofs, st)) != cudaSuccess) return e;
-  if ((e = launch_g2p2g(s, x, v.ap, ndofs, dt, nullptr, st)) != cudaSuccess) return e;
+  if ((e = launch_g2p2g(s, x, v.ap, ndofs, dt, st)) != cudaSuccess) return e;
   k_cg_start<<<cg_grid(ndofs), kThreads, 0, st>>>(s, x, b, v, ndofs, dt, cs, tol, rel_tol, max_iters);
   return cudaGetLastError();
 }
@@ -3331,8 +3230,9 @@ cudaError_t launch_cg_begin(scene_device &s, const float *x, const float *b, con
 cudaError_t launch_cg_iteration(scene_device &s, float *x, const cg_vectors &v, long long ndofs, float dt,
                                 cg_state *cs, int max_iters, cudaStream_t st) {
   const int grid = cg_grid(ndofs);
-  // its work counter was cleared by the pass before
-  k_g2p2g<<<num_sms() * 2, kG2P2GThreads, kG2P2GSmem, st>>>(s, v.p, v.ap, ndofs, dt, &cs->done);
+  // (its work counters were cleared by the pass before)
+  const cudaError_t e = launch_force(s, v.p, v.ap, ndofs, dt, &cs->done, st);
+  if (e != cudaSuccess) return e;
   k_cg_apply<<<grid, kThreads, 0, st>>>(s, v, ndofs, dt, cs);
   k_cg_update<<<grid, kThreads, 0, st>>>(s, x, v, ndofs, cs, max_iters);
   k_cg_direction<<<grid, kThreads, 0, st>>>(s, v, ndofs, cs);
