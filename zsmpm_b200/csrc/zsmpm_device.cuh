@@ -321,6 +321,10 @@ __device__ __forceinline__ bool svd3_columns(const float *A, float *U, float *S,
   V[1] = xy + wz;
   V[5] = yz + wx;
   V[6] = zx + wy;
+  // V's columns have length 1 + e: the normalisation above rounds near 1, the same way for most
+  // particles, so e is a bias of about 8e-8.  The singular values are freed of it, or the strain
+  // of a committed F would take it twice a substep.
+  const float e = fmaf(qs, qs, -1.f) + fmaf(qx, qx, fmaf(qy, qy, zz));
   float lo = 3.4e38f, hi = 0.f;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -333,7 +337,8 @@ __device__ __forceinline__ bool svd3_columns(const float *A, float *U, float *S,
     const float r = fmaf(0.5f * y, fmaf(-q, y, 1.f), y);
     lo = fminf(lo, rho);
     hi = fmaxf(hi, rho);
-    S[c] = fmaf(0.5f * y, fmaf(-q, q, rho), q);
+    const float len = fmaf(0.5f * y, fmaf(-q, q, rho), q);
+    S[c] = fmaf(-e, len, len);
     U[3 * c] = b0 * r;
     U[3 * c + 1] = b1 * r;
     U[3 * c + 2] = b2 * r;
