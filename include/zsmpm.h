@@ -473,10 +473,11 @@ typedef struct {
   int32_t g2p_threads;      /* G2P CTA size: 128 or 256 (0 = default 256) */
   int32_t g2p_ctas_per_sm;  /* persistent G2P CTAs per SM, 1-6 (0 = default: 3, learned 2) */
   int32_t p2g_ctas_per_sm;  /* persistent P2G CTAs per SM, 1-4 (0 = the staging depth's
-                               default: 4 for 8 ranks, 3 for 12, 2 for 16) */
+                               default: 4 for 8 ranks, 3 for 12, 2 for 16; at most 3 where
+                               p2g_ranks is 0) */
   float g2p_ms, p2g_ms;     /* stage times of the chosen shapes (autotune output) */
-  int32_t p2g_ranks;        /* P2G staging depth: particles per cell staged per round, 8, 12 or
-                               16 (0 = 12); deeper staging means fewer rounds on dense cells and
+  int32_t p2g_ranks;        /* P2G staging depth: particles per cell in a warp's ring, 8, 12 or
+                               16 (0 = 8); deeper staging keeps more copies in flight and takes
                                more shared memory per CTA */
 } zsmpm_tuning;
 

@@ -399,10 +399,6 @@ ZSMPM_API zsmpm_status zsmpm_scene_create(const zsmpm_scene_desc *desc, zsmpm_sc
   scene_params &p = s->dev.prm;
   p.dx = desc->dx;
   p.inv_dx = 1.f / desc->dx;
-  {
-    int ex = 0;
-    p.dx_pow2 = std::isfinite(desc->dx) && desc->dx > 0.f && std::frexp(desc->dx, &ex) == 0.5f ? 1 : 0;
-  }
   p.dt = desc->dt;
   p.kappa = desc->dt * (4.f * p.inv_dx * p.inv_dx);  // dt * D_inv (P2G.hpp:52, :104)
   p.four_over_dx = 4.f * p.inv_dx;
@@ -1302,7 +1298,7 @@ ZSMPM_API zsmpm_status zsmpm_autotune(zsmpm_scene *s, int32_t trials, zsmpm_tuni
       }
     }
   // P2G: staging depth x CTAs per SM, up to what the depth's shared memory lets stay resident
-  // (8 ranks: 55 KB, 4 CTAs; 12: 72 KB, 3; 16: 88 KB, 2)
+  // (8 ranks: 4 CTAs, 12: 3, 16: 2)
   float best_p2g = 3.4e38f;
   const int p2g_shapes[6][2] = {{12, 3}, {12, 2}, {8, 4}, {8, 3}, {16, 2}, {16, 1}};
   if (st == ZSMPM_OK)
@@ -1341,6 +1337,7 @@ ZSMPM_API zsmpm_status zsmpm_set_tuning(zsmpm_scene *s, const zsmpm_tuning *t) {
       (t->p2g_ranks != 0 && t->p2g_ranks != 8 && t->p2g_ranks != 12 && t->p2g_ranks != 16))
     return fail(ZSMPM_ERR_INVALID_ARG, "tuning out of range");
   // more CTAs than the staging depth's shared memory lets stay resident would queue, not run
+  // (a CTA count without a depth is held to three)
   const int ranks = t->p2g_ranks ? t->p2g_ranks : 12;
   const int max_p2g = ranks == 8 ? 4 : ranks == 12 ? 3 : 2;
   if (t->p2g_ctas_per_sm > max_p2g)
