@@ -228,9 +228,9 @@ def g2p_algorithmic_bytes(n: int, nb: int, plastic: bool) -> int:
 
 
 def g2p_implementation_bytes(n: int, nb: int, plastic: bool) -> int:
-    """What this k_g2p actually moves per launch: per particle reads slot index 4, x|m 16,
-    F 36, id 4 (+ plastic 4) and writes x|m 16, v 16 (float4), C 36, A 36, F 36, id 4
-    (+ plastic 4), plus the same 12 B per block cell."""
+    """What k_g2p moves per launch at most: per particle reads slot index 4, x|m 16, F 36, id 4
+    (+ plastic 4) and writes x|m 16, v and A 52 (48 as its three float4 rows), C 36 (the last
+    substep of a run only), F 36, id 4 (+ plastic 4), plus the same 12 B per block cell."""
     per_particle = 4 + 16 + 36 + 4 + 16 + 16 + 36 + 36 + 36 + 4 + (8 if plastic else 0)
     return n * per_particle + nb * 512 * 12
 
